@@ -289,14 +289,17 @@ qesb_status qesb_autotune_batch(qesb_handle *const *handles, int n, int *best, f
  *   "pdl"                1 = z-march list sweeps and window checks as programmatic dependent launches,
  *                        each grid's CTAs scheduled while the previous grid finishes; 0 = off (default:
  *                        inside the CUDA-graph chunks it measured 0.6 % slower on the headline batch)
- *   "variant"            sweep variant index (-1 = autotuned / default), see qesb_num_variants
+ *   "variant"            sweep variant index, see qesb_num_variants (-1 = the solver's choice: a domain whose
+ *                        lambda fits the chip's shared memory, up to about 5 million cells, is solved by one
+ *                        cooperative launch with lambda resident there; others run the autotuned / default shape)
  *   "batch_variant"      sweep shape for qesb_solve_batch led by this handle (-1 = from "variant");
  *                        set by qesb_autotune_batch
  *   "autotune"           1 = run qesb_autotune at the first solve of an untuned grid shape (default 0)
  *   "wait_limit"         polls of a staged sweep's shared-memory stage barrier before the kernel gives
  *                        up, lets its copies in flight land, and the solve returns QESB_ERR_CUDA
  *                        ("sweep stage wait gave up"); 0 = the default (2^22 polls). Applies to the
- *                        bulk-copy sweep shapes and to batches led by this handle */
+ *                        bulk-copy sweep shapes, the resident kernel's waits for its other CTAs, and
+ *                        batches led by this handle */
 qesb_status qesb_set_tolerance(qesb_handle *h, float tol);
 qesb_status qesb_set_option(qesb_handle *h, const char *key, int value);
 /* cudaStream_t to run on (NULL = the handle's own stream). */

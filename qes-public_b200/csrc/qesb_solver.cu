@@ -41,6 +41,7 @@
 #include "qesb_sor_tiled.cuh"
 #include "qesb_sor_split.cuh"
 #include "qesb_sor_zm.cuh"
+#include "qesb_sor_res.cuh"
 #include "qesb_wall_log.cuh"
 #include "qesb_fp64.cuh"
 #include "qesb_sor_bulk.cuh"
@@ -837,6 +838,14 @@ struct SweepGraph {
   }
 };
 
+// Tiles of a resident solve (qesb_sor_res.cu) over at most so many CTAs, with the
+// estimated cycles of a half-sweep; nty = 0: the domain does not fit.
+struct ResPlan {
+  int nty = 0, ntz = 0;
+  int tym = 0, tzm = 0;  // the largest tile
+  double cost = 0;
+};
+
 struct qesb_handle {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -934,6 +943,23 @@ struct qesb_handle {
   SweepCtl *h_ctl = nullptr, *h_ctl_dev = nullptr;  // mapped pinned, and its device alias
   unsigned char *h_io = nullptr, *h_io_dev = nullptr;  // mapped pinned scratch for small reads (kIoBytes)
   SweepGraph sgraph;  // iteration-loop graph of the sweep kernels
+
+  // resident solves: the loop states of the start stage and the pre-phase (d_state holds the reference loop's),
+  // their error histories, the domain's barrier block, and the descriptors of launches led by this handle
+  SolveState *d_rstate = nullptr;  // [2]: pre-phase, start stage (behind d_state; the host's behind h_state)
+  SolveState *h_rstate = nullptr, *h_rstate_dev = nullptr;
+  double *d_rerr = nullptr;
+  int rerr_cap = 0;
+  ResSync *d_rsync = nullptr;
+  struct ResList {
+    unsigned char *blk = nullptr, *stage = nullptr, *stage_dev = nullptr;
+    int cap = 0;
+    // the tiles' exchange buffer and the number of the last half-sweep its marks may carry
+    unsigned char *xbuf = nullptr;
+    size_t xbytes = 0;
+    unsigned long long epoch = 0;
+    std::map<std::tuple<int, int, int, int>, ResPlan> plans;  // by grid and CTAs
+  } rlist;
 
   // iteration-loop graphs of the tiled path, one per (variant, starting buffer)
   struct GraphKey {
@@ -1742,6 +1768,436 @@ qesb_status run_iterations_sweep(qesb_handle *h, const SweepVariant &sv, int ite
   return QESB_OK;
 }
 
+// ---------------------------------------------------------------------------
+// resident solves (qesb_sor_res.cuh)
+// ---------------------------------------------------------------------------
+constexpr int kResThreads = 512;         // one CTA per SM
+constexpr int kResSmemBytes = 230400;    // the per-block limit less the kernel's static part
+constexpr int kResMaxLaunches = 16;           // launches of one batch (group sizes)
+
+__global__ void k_res_stamp(ResCtl *ctl) { ctl->t0 = global_ns(); }
+
+// lambda and R of the padded layout into the split layout, one pass.
+__global__ void k_res_to_split(DevGrid G, SplitGeom S, const float *__restrict__ lam, const float *__restrict__ R,
+                               float *__restrict__ lam_s, float *__restrict__ R_s)
+{
+  const int j = blockIdx.y, k = blockIdx.z;
+  for (int i = threadIdx.x + blockIdx.x * blockDim.x; i < G.X; i += gridDim.x * blockDim.x) {
+    const long d = ((i + j + k) & 1) * S.CS + S.row(j, k, G.Y) + (i >> 1), p = G.pad(i, j, k);
+    lam_s[d] = lam[p];
+    R_s[d] = R[p];
+  }
+}
+
+// lambda after a resident solve of at least one iteration back into the padded
+// layout; the ground plane takes plane 1's values, as every iteration's mirror
+// leaves it. Nothing is written when a phase before the reference loop (pre:
+// the states of the two) met a NaN or the launch gave up: the handle keeps its
+// start.
+__global__ void k_res_to_pad(DevGrid G, SplitGeom S, const float *__restrict__ src, float *__restrict__ dst,
+                             const SolveState *__restrict__ pre, const ResCtl *__restrict__ ctl)
+{
+  if (pre[0].nan || pre[1].nan || ctl->fault) return;
+  const int j = blockIdx.y, k = blockIdx.z, ks = k == 0 ? 1 : k;
+  for (int i = threadIdx.x + blockIdx.x * blockDim.x; i < G.X; i += gridDim.x * blockDim.x)
+    dst[G.pad(i, j, k)] = src[((i + j + ks) & 1) * S.CS + S.row(j, ks, G.Y) + (i >> 1)];
+}
+
+// The estimate: row steps of the CTA's warps (350 cycles for all of them, dearer
+// where R streams from L2) and the exchange. Measured solves take 1.45 (the
+// smallest domains) to 1.95 times it: 1.85, at 1.9 GHz, in kResUs.
+constexpr double kResUs = 2 * 1.85 / 1900.0;  // microseconds an iteration per estimated cycle of a half-sweep
+ResPlan res_plan(const DevGrid &G, int ctas)
+{
+  constexpr int NW = kResThreads / 32;
+  ResPlan best;
+  const int nq4 = ((G.X + 1) / 2 + 3) / 4, P = 4 * nq4, rows = G.Y - 2, planes = G.Z - 2;
+  const long cap = kResSmemBytes / 4;
+  // for each cut along z the most tiles along y that the CTAs allow (no more than their row count needs)
+  for (int ntz = 1; ntz <= std::min(planes, ctas); ++ntz) {
+    const int tz = (planes + ntz - 1) / ntz, ty = (rows + std::min(rows, ctas / ntz) - 1) / std::min(rows, ctas / ntz);
+    const int nty = (rows + ty - 1) / ty;
+    const long base = 2048 + 72L * tz + 2L * (tz + 2) * (ty + 2) * P + 2L * tz * ty * nq4 + 4L * (tz + ty) * nq4 + 8;
+    if (base > cap) continue;
+    const int rp = (int)std::min<long>(tz, (cap - base) / (2L * ty * P));
+    const int ch = ((tz + 1) / 2 * nq4 + 31) / 32 + (tz / 2 * nq4 + 31) / 32;  // warps' columns
+    int steps = 1 << 30;
+    for (int n = 1; n <= std::min(ty, 32); ++n) steps = std::min(steps, (ch * n + NW - 1) / NW * ((ty + n - 1) / n + 4));
+    const double step = 350.0 * (1.0 + 0.4 * (tz - rp) / tz);
+    const double comm = nty * ntz > 1 ? 2000.0 + 0.25 * (tz + ty) * nq4 : 200.0;
+    const double cost = step * steps + comm;
+    if (best.nty == 0 || cost < best.cost) {
+      best.nty = nty;
+      best.ntz = ntz;
+      best.cost = cost;
+      best.tym = ty;
+      best.tzm = tz;
+    }
+  }
+  return best;
+}
+
+int sm_count(int device)
+{
+  static int nsm[64] = {};
+  int &v = nsm[device & 63];
+  if (!v) {
+    int n = 0;
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device);
+    v = n;
+  }
+  return v;
+}
+int res_ctas(int device) { return sm_count(device); }
+
+// Half-sweep numbers a domain's solve may use.
+unsigned long long res_halves(const qesb_handle *h, int itermax)
+{
+  return 2ull * ((unsigned long long)itermax + (prephase_on(h) ? h->pre_iters : 0) + (start_on(h) ? h->start_iters : 0) + 1);
+}
+
+const ResPlan &res_plan_of(qesb_handle *lead, const DevGrid &G, int ctas)
+{
+  auto &m = lead->rlist.plans;
+  const std::tuple<int, int, int, int> key(G.X, G.Y, G.Z, ctas);
+  auto it = m.find(key);
+  if (it == m.end()) {
+    if (m.size() > 4096) m.clear();
+    it = m.emplace(key, res_plan(G, ctas)).first;
+  }
+  return it->second;
+}
+
+// Whether a solve of h led by `lead` may take the resident kernel: no sweep
+// shape asked for, lambda fits the chip's shared memory, and the half-sweeps it
+// may run fit *room, the numbers left in the exchange buffer's 32-bit marks (a
+// batch's domains share them). A lone domain that may does: it is 1.5 to 2.2
+// times as fast as the best streaming shape at every size that fits (us an
+// iteration, resident / streaming: 40 x 40 x 20 5.7 / 9.4, 100 x 100 x 50
+// 7.7 / 13.0, 200 x 180 x 60 10.0 / 18.6, 256 x 256 x 64 14.0 / 21.0).
+constexpr unsigned long long kResMarks = 0xf0000000ull;
+bool res_may(qesb_handle *lead, const qesb_handle *h, int itermax, unsigned long long *room)
+{
+  if (itermax <= 0 || lead->opt_variant >= 0 || lead->opt_k != 0) return false;
+  const unsigned long long need = res_halves(h, itermax);
+  if (need > *room || res_plan_of(lead, h->G, res_ctas(lead->device)).nty == 0) return false;
+  *room -= need;
+  return true;
+}
+
+// The launches of a list of domains: domains of about the same best group size
+// go together, large ones first.
+struct ResLaunch {
+  int first, n, groups, gsz;  // of `order`
+};
+struct ResSchedule {
+  std::vector<int> order;
+  std::vector<ResLaunch> launches;
+  double cost = 0;           // estimated cycles of a half-sweep of all domains
+  std::vector<double> each;  // a domain's own share of it
+};
+ResSchedule res_schedule(qesb_handle *lead, const std::vector<qesb_handle *> &hs)
+{
+  const int n = (int)hs.size(), sms = res_ctas(lead->device);
+  ResSchedule r;
+  r.order.resize(n);
+  r.each.resize(n);
+  std::vector<int> ng(n);
+  for (int i = 0; i < n; ++i) {
+    r.order[i] = i;
+    for (int g = 1; g <= std::min(n, sms); ++g) {
+      const ResPlan &p = res_plan_of(lead, hs[i]->G, sms / g);
+      if (!p.nty) break;
+      if (ng[i] == 0 || p.cost / g < r.each[i]) {
+        r.each[i] = p.cost / g;
+        ng[i] = g;
+      }
+    }
+  }
+  std::stable_sort(r.order.begin(), r.order.end(), [&](int a, int b) {
+    if (ng[a] != ng[b]) return ng[a] < ng[b];
+    return hs[a]->G.XY * hs[a]->G.Z > hs[b]->G.XY * hs[b]->G.Z;
+  });
+  // the time of one launch of order[i, j) in g groups: each takes the next domain when it is free
+  auto span = [&](int i, int j, int g) {
+    std::vector<double> t(g, 0.0);
+    for (int q = i; q < j; ++q) {
+      const ResPlan &p = res_plan_of(lead, hs[r.order[q]]->G, sms / g);
+      if (!p.nty) return -1.0;
+      *std::min_element(t.begin(), t.end()) += p.cost;
+    }
+    return *std::max_element(t.begin(), t.end());
+  };
+  auto best_launch = [&](int i, int j, double *cost) {
+    ResLaunch l{i, j - i, 1, sms};
+    *cost = span(i, j, 1);
+    for (int g = 2; g <= std::min(j - i, sms); ++g) {
+      const double c = span(i, j, g);
+      if (c < 0) break;
+      if (c < *cost) {
+        *cost = c;
+        l.groups = g;
+        l.gsz = sms / g;
+      }
+    }
+    return l;
+  };
+  for (int i = 0; i < n;) {
+    int j = i;
+    while (j < n && ng[r.order[j]] == ng[r.order[i]]) ++j;
+    double c = 0;
+    ResLaunch l = best_launch(i, j, &c);
+    if (!r.launches.empty()) {  // together with the launch before where that is shorter (or there are many)
+      const ResLaunch &b = r.launches.back();
+      double cb = 0, cm = 0;
+      const ResLaunch before = best_launch(b.first, i, &cb), m = best_launch(b.first, j, &cm);
+      (void)before;
+      if (cm <= cb + c || (int)r.launches.size() == kResMaxLaunches) {
+        r.launches.back() = m;
+        r.cost += cm - cb;
+        i = j;
+        continue;
+      }
+    }
+    r.launches.push_back(l);
+    r.cost += c;
+    i = j;
+  }
+  return r;
+}
+
+// Microseconds that a domain adds to an iteration of the streaming list sweeps
+// (measured: 3.0 a million cells on full 128-cell row tiles, 4.5 where half of a
+// tile is empty), and what the list's launches take of themselves.
+double list_us(const DevGrid &G)
+{
+  const int qn = (G.X + 1) / 2;
+  return 3.0e-6 * (double)G.XY * G.Z * 0.5 * (1.0 + 128.0 * ((qn + 127) / 128) / qn);
+}
+constexpr double kListUs = 12.0;
+
+// Which domains of a batch take the resident kernel, of those that may: all,
+// none, or those it is faster for than their part of the list sweeps, by the
+// shorter estimate. A list of small domains gains the most (16 of 64 x 64 x 32:
+// 10 against 35 us an iteration; 16 of 128 x 128 x 48: 42 against 76), many
+// large ones (16 of 192 x 192 x 64: 171 against 133) stay with the list sweeps.
+std::vector<char> res_choose(qesb_handle *lead, qesb_handle *const *hs, int n, const std::vector<char> &may)
+{
+  std::vector<qesb_handle *> all;
+  std::vector<int> of;
+  double others = 0;  // list time of the domains that have no choice
+  for (int i = 0; i < n; ++i) {
+    if (may[i]) {
+      all.push_back(hs[i]);
+      of.push_back(i);
+    } else {
+      others += list_us(hs[i]->G);
+    }
+  }
+  std::vector<char> none(n, 0);
+  if (all.empty()) return none;
+  const ResSchedule sch = res_schedule(lead, all);
+  double list_all = 0, list_rest = 0;
+  std::vector<char> some(n, 0);
+  std::vector<qesb_handle *> part;
+  for (size_t q = 0; q < all.size(); ++q) {
+    const double l = list_us(all[q]->G);
+    list_all += l;
+    if (kResUs * sch.each[q] < l) {
+      some[of[q]] = 1;
+      part.push_back(all[q]);
+    } else {
+      list_rest += l;
+    }
+  }
+  const auto list = [&](double us) { return us + others > 0 ? us + others + kListUs : 0.0; };
+  const double t_all = kResUs * sch.cost + list(0.0), t_none = list(list_all);
+  const double t_some = part.empty() ? t_none : kResUs * res_schedule(lead, part).cost + list(list_rest);
+  if (t_none <= t_all && t_none <= t_some) return none;
+  return t_all <= t_some ? may : some;
+}
+
+qesb_status res_prepare(qesb_handle *h)
+{
+  const int need = (prephase_on(h) ? h->pre_iters : 0) + (start_on(h) ? h->start_iters : 0);
+  if (need > h->rerr_cap) {
+    if (h->d_rerr) cudaFree(h->d_rerr);
+    h->d_rerr = nullptr;
+    h->rerr_cap = 0;
+    CKS(dalloc(&h->d_rerr, (size_t)need));
+    h->rerr_cap = need;
+  }
+  return QESB_OK;
+}
+
+// Solves the handles' domains (R computed, err and state zeroed on s) from their current lambda to the end of their reference loops:
+// one cooperative launch per group size. Enqueues everything on s, the final
+// states' copies to the mapped buffers included; the caller waits and then
+// calls res_finish. *launches: kernels launched.
+qesb_status res_enqueue(qesb_handle *lead, const std::vector<qesb_handle *> &hs, int itermax, cudaStream_t s,
+                        int *launches)
+{
+  const int n = (int)hs.size(), sms = res_ctas(lead->device);
+  WordBatch wb(s);
+  const ResSchedule sch = res_schedule(lead, hs);
+  const std::vector<int> &order = sch.order;
+  const std::vector<ResLaunch> &ls = sch.launches;
+  // descriptors: [launch controls][group slots][domains]
+  const size_t o_slot = sizeof(ResCtl) * kResMaxLaunches,
+               o_dom = o_slot + sizeof(unsigned long long) * (size_t)kResMaxLaunches * sms;
+  qesb_handle::ResList &L = lead->rlist;
+  if (L.cap < n) {
+    if (L.blk) cudaFree(L.blk);
+    if (L.stage) cudaFreeHost(L.stage);
+    L.blk = L.stage = nullptr;
+    L.cap = 0;
+    const size_t bytes = o_dom + sizeof(ResDomain) * (size_t)n;
+    CK(cudaMalloc((void **)&L.blk, bytes));
+    CKS(host_mapped(&L.stage, &L.stage_dev, bytes));
+    L.cap = n;
+  }
+  std::memset(L.stage, 0, o_dom);
+  // the exchange buffer: room for the largest launch, zeroed when (re)allocated and before its 32-bit marks wrap
+  std::vector<ResPlan> plans(n);
+  std::vector<int> xstride(ls.size(), 0);
+  size_t xneed = 0;
+  unsigned long long halves = 0;
+  for (size_t l = 0; l < ls.size(); ++l) {
+    for (int q = ls[l].first; q < ls[l].first + ls[l].n; ++q) {
+      const qesb_handle *h = hs[order[q]];
+      plans[q] = res_plan_of(lead, h->G, ls[l].gsz);
+      xstride[l] = std::max(xstride[l], 2 * (plans[q].tym + plans[q].tzm) * (((h->G.X + 1) / 2 + 3) / 4));
+      halves += res_halves(h, itermax);
+    }
+    xneed = std::max(xneed, (size_t)ls[l].groups * 2 * ls[l].gsz * xstride[l] * 32);
+  }
+  if (L.xbytes < xneed) {
+    if (L.xbuf) cudaFree(L.xbuf);
+    L.xbuf = nullptr;
+    L.xbytes = 0;
+    CK(cudaMalloc((void **)&L.xbuf, xneed));
+    L.xbytes = xneed;
+    L.epoch = ~0ull;
+  }
+  if (L.epoch == ~0ull || L.epoch + halves >= 0xffffff00ull) {
+    CK(zero_async(L.xbuf, L.xbytes, s));
+    L.epoch = 0;
+  }
+  ResDomain *doms = reinterpret_cast<ResDomain *>(L.stage + o_dom);
+  for (const ResLaunch &l : ls)
+    for (int q = l.first; q < l.first + l.n; ++q) {
+      qesb_handle *h = hs[order[q]];
+      const DevGrid &G = h->G;
+      const ResPlan &p = plans[q];
+      ResDomain d{};
+      d.X = G.X;
+      d.Y = G.Y;
+      d.Z = G.Z;
+      d.PQ = h->S.PQ;
+      d.CS = h->S.CS;
+      d.nty = p.nty;
+      d.ntz = p.ntz;
+      d.nq4 = ((G.X + 1) / 2 + 3) / 4;
+      d.magic = (unsigned)(((1ull << 32) + d.nq4 - 1) / d.nq4);
+      d.tym = p.tym;
+      d.tzm = p.tzm;
+      d.epoch = (unsigned)L.epoch;
+      L.epoch += res_halves(h, itermax);
+      d.lam = h->d_lam_s;
+      d.R = h->d_R_s;
+      d.mask = h->d_mask_s;
+      d.val = h->d_val;
+      d.snap = h->d_snap;
+      d.wtol = h->win_tol;
+      d.sync = h->d_rsync;
+      // the padded copies of the coefficients, which only the full-coefficient sweep reads, hold the lists of wall
+      // cells meanwhile: 8 bytes x 4 nq4 <= (X + 8) / 2 cells a row, within their 4 bytes x (X + 16)
+      for (int c = 0; c < 2; ++c) d.walls[c] = reinterpret_cast<uint2 *>(h->d_pc[c]);
+      h->pc_ready = false;
+      SweepDomain sd;
+      if (start_on(h)) {
+        CKS(sweep_domain_start(h, sd, s));
+        d.ph[d.nph++] = {sd.inv, h->d_rerr + h->pre_iters, h->d_rstate + 1, sd.tol, sd.c1, sd.itermax, 0};
+      }
+      if (prephase_on(h)) {
+        CKS(sweep_domain_pre(h, sd, s));
+        d.ph[d.nph++] = {sd.inv, h->d_rerr, h->d_rstate, sd.tol, sd.c1, sd.itermax, 0};
+      }
+      sd = sweep_domain(h, itermax, (double)h->tol);
+      d.ph[d.nph++] = {sd.inv, h->d_err, h->d_state, sd.tol, sd.c1, sd.itermax, sd.wK};
+      std::memcpy(&doms[q], &d, sizeof d);
+      CKS(wb.zero(h->d_rsync, sizeof(ResSync)));
+      CKS(wb.zero(h->d_rstate, 2 * sizeof(SolveState)));
+      if (h->rerr_cap) CKS(wb.zero(h->d_rerr, sizeof(double) * (size_t)h->rerr_cap));
+    }
+  CKS(wb.flush());
+  for (qesb_handle *h : hs)
+    k_res_to_split<<<row_grid(h->G, h->G.Y, h->G.Z, h->G.X), 256, 0, s>>>(h->G, h->S, h->d_lam, h->d_R, h->d_lam_s,
+                                                                         h->d_R_s);
+  CKS(copy_words(L.blk, L.stage_dev, o_dom + sizeof(ResDomain) * (size_t)n, s));
+  k_res_stamp<<<1, 1, 0, s>>>(reinterpret_cast<ResCtl *>(L.blk));
+  CK(cudaEventRecord(lead->evs[0], s));
+  for (size_t q = 0; q < ls.size(); ++q) {
+    ResArgs a{};
+    a.dom = reinterpret_cast<ResDomain *>(L.blk + o_dom) + ls[q].first;
+    a.n = ls[q].n;
+    a.gsz = ls[q].gsz;
+    a.ctl = reinterpret_cast<ResCtl *>(L.blk) + q;
+    a.slot = reinterpret_cast<unsigned long long *>(L.blk + o_slot) + q * sms;
+    a.xbuf = reinterpret_cast<ulonglong2 *>(L.xbuf);
+    a.xstride = xstride[q];
+    a.wait_limit = lead->opt_wait_limit;
+    a.smem_floats = kResSmemBytes / 4;
+    CK(res_launch(a, ls[q].groups, kResThreads, s));
+  }
+  CK(cudaEventRecord(lead->evs[1], s));
+  for (size_t l = 0; l < ls.size(); ++l)
+    for (int q = ls[l].first; q < ls[l].first + ls[l].n; ++q) {
+      qesb_handle *h = hs[order[q]];
+      k_res_to_pad<<<row_grid(h->G, h->G.Y, h->G.Z, h->G.X), 256, 0, s>>>(
+          h->G, h->S, h->d_lam_s, h->d_lam, h->d_rstate, reinterpret_cast<ResCtl *>(L.blk) + l);
+      CKS(wb.add(h->h_rstate_dev, h->d_rstate, 2 * sizeof(SolveState)));
+    }
+  CK(cudaGetLastError());
+  CKS(wb.add(L.stage_dev, L.blk, o_slot));  // the launches' controls, back into the staging image
+  CKS(wb.flush());
+  *launches = (int)ls.size() + 2 * n + 4;
+  return QESB_OK;
+}
+
+// After the stream has drained: faults and NaNs of the launch, the iteration
+// counts of the phases before the reference loop. `batch`: index in messages.
+qesb_status res_finish(qesb_handle *lead, const std::vector<qesb_handle *> &hs, const std::vector<int> &index,
+                       bool batch, unsigned long long *t0)
+{
+  const ResCtl *ctl = reinterpret_cast<const ResCtl *>(lead->rlist.stage);
+  if (t0) *t0 = ctl->t0;
+  for (int q = 0; q < kResMaxLaunches; ++q)
+    if (ctl[q].fault) return qesb_fail(QESB_ERR_CUDA, "sweep stage wait gave up");
+  char where[48] = "";
+  for (size_t i = 0; i < hs.size(); ++i) {
+    qesb_handle *h = hs[i];
+    if (batch) snprintf(where, sizeof where, " of batch domain %d", index[i]);
+    if (start_on(h) && h->h_rstate[1].nan)
+      return qesb_fail(QESB_ERR_NUMERIC, "NaN in lambda%s during the pre-phase's start stage", where);
+    if (prephase_on(h) && h->h_rstate[0].nan)
+      return qesb_fail(QESB_ERR_NUMERIC, "NaN in lambda%s during the pre-phase", where);
+    h->last_pre_iterations = (start_on(h) ? h->h_rstate[1].it : 0) + (prephase_on(h) ? h->h_rstate[0].it : 0);
+  }
+  return QESB_OK;
+}
+
+// One solve on the resident kernel: as run_iterations_sweep, in one launch.
+qesb_status run_iterations_resident(qesb_handle *h, int itermax)
+{
+  cudaStream_t s = h->stream;
+  CKS(res_prepare(h));
+  CKS(res_enqueue(h, {h}, itermax, s, &h->last_launches));
+  for (int q = 2; q < 4; ++q) CK(cudaEventRecord(h->evs[q], s));  // one launch runs every phase: evs[0..1]
+  h->sweeps_timed = true;
+  return QESB_OK;
+}
+
 // FP64 final divergence check of (u, v, w) into h->d_div (all three needed).
 qesb_status enqueue_divergence_check(qesb_handle *h, const float *u, const float *v, const float *w, cudaStream_t s)
 {
@@ -1773,7 +2229,9 @@ qesb_status solve_impl(qesb_handle *h, int itermax, float *u, float *v, float *w
   CK(zero_async(h->d_state, sizeof(SolveState), s));
   CK(cudaEventRecord(h->ev[1], s));
   const bool packed = h->packed && h->opt_path == 1;
-  if (packed && h->opt_autotune && h->opt_variant < 0 && tuned_variant(G) < 0) {
+  unsigned long long room = kResMarks;
+  const bool resident = packed && res_may(h, h, itermax, &room);
+  if (packed && !resident && h->opt_autotune && h->opt_variant < 0 && tuned_variant(G) < 0) {
     CKS(qesb_autotune(h, nullptr, nullptr, 0));
     CK(cudaEventRecord(h->ev[1], s));
   }
@@ -1781,12 +2239,13 @@ qesb_status solve_impl(qesb_handle *h, int itermax, float *u, float *v, float *w
   // the fused tiled kernels have no window checks and no pre-phase: either runs on the sweep kernels
   if (packed && (h->win_k > 0 || prephase_on(h)) && vi < kSplitVariant) vi = kSplitVariant + kDefaultSweep;
   const bool split = packed && vi >= kSplitVariant;
-  const Variant *var = packed && !split ? &kVariants[vi] : nullptr;
+  const Variant *var = packed && !split && !resident ? &kVariants[vi] : nullptr;
   h->last_launches = 0;
   h->last_pre_iterations = 0;
   h->sweeps_timed = false;
   if (itermax > 0) {
-    if (split) CKS(run_iterations_sweep(h, kSweepVariants[vi - kSplitVariant], itermax));
+    if (resident) CKS(run_iterations_resident(h, itermax));
+    else if (split) CKS(run_iterations_sweep(h, kSweepVariants[vi - kSplitVariant], itermax));
     else if (var) CKS(run_iterations_tiled(h, *var, itermax));
     else CKS(run_iterations_full(h, itermax));
   }
@@ -1802,6 +2261,7 @@ qesb_status solve_impl(qesb_handle *h, int itermax, float *u, float *v, float *w
   if (check) CKS(copy_words(h->h_io_dev, h->d_div, sizeof(double), s));
   CKS(copy_words(h->h_state_dev, h->d_state, sizeof(SolveState), s));
   CK(cudaStreamSynchronize(s));
+  if (resident) CKS(res_finish(h, {h}, {0}, false, nullptr));
   if (check) std::memcpy(&div, h->h_io, sizeof div);
   if (st) {
     st->max_divergence = div;
@@ -1862,7 +2322,7 @@ void free_all(qesb_handle *h)
                   h->d_own_in[2], h->d_own_in[3], h->d_own_in[4], h->d_own_in[5], h->d_own_flag,
                   h->d_own_u0, h->d_own_v0, h->d_own_w0, h->d_dz, h->d_vmax, h->d_inv, h->d_val,
                   h->d_inv_pre, h->d_inv_start, h->d_bad, h->d_err, h->d_state, h->d_u, h->d_v, h->d_w, h->d_wbits,
-                  h->d_wcut, h->d_snap, h->d_tmaps};
+                  h->d_wcut, h->d_snap, h->d_tmaps, h->d_rerr, h->rlist.blk, h->rlist.xbuf};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   h->list.destroy();
@@ -1870,6 +2330,7 @@ void free_all(qesb_handle *h)
   h->bgraph_start.reset();
   h->bgraph_pre.reset();
   h->bgraph.reset();
+  if (h->rlist.stage) cudaFreeHost(h->rlist.stage);
   if (h->h_state) cudaFreeHost(h->h_state);
   if (h->h_ctl) cudaFreeHost(h->h_ctl);
   if (h->h_io) cudaFreeHost(h->h_io);
@@ -1941,11 +2402,20 @@ qesb_status qesb_create(const qesb_grid *grid, float tol, int device, qesb_handl
   TRY(dalloc(&h->d_inv_start, 64 * G.Z));
   TRY(dalloc(&h->d_val, 6 * G.Z));
   TRY(dalloc(&h->d_bad, 1));
-  TRY(dalloc(&h->d_state, 1));
+  // the loop states (reference loop, pre-phase, start stage) and the resident kernel's barrier block, aligned
+  static_assert(sizeof(ResSync) % sizeof(long) == 0 && alignof(ResSync) <= 256, "one allocation for both");
+  constexpr size_t o_sync = (3 * sizeof(SolveState) + 255) / 256 * 256;
+  unsigned char *st_blk = nullptr;
+  TRY(dalloc(&st_blk, o_sync + sizeof(ResSync)));
+  h->d_state = reinterpret_cast<SolveState *>(st_blk);
+  h->d_rstate = h->d_state + 1;
+  h->d_rsync = reinterpret_cast<ResSync *>(st_blk + o_sync);
   TRY(dalloc(&h->d_div, 1));
   TRY(h->list.create(1));
   TRY(ensure_err(h, 1024));
-  TRY(host_mapped(&h->h_state, &h->h_state_dev, sizeof(SolveState)));
+  TRY(host_mapped(&h->h_state, &h->h_state_dev, 3 * sizeof(SolveState)));
+  h->h_rstate = h->h_state + 1;
+  h->h_rstate_dev = h->h_state_dev + 1;
   TRY(host_mapped(&h->h_ctl, &h->h_ctl_dev, sizeof(SweepCtl)));
   TRY(host_mapped(&h->h_io, &h->h_io_dev, kIoBytes));
   for (auto &e : h->ev)
@@ -2491,7 +2961,22 @@ qesb_status qesb_solve_batch(qesb_handle *const *hs, int n, int itermax, float *
   if (vi < kSplitVariant) vi = kSplitVariant + kDefaultSweep;
   const SweepVariant &sv = kSweepVariants[vi - kSplitVariant];
   CK(cudaEventRecord(h0->ev[0], s));
-  std::vector<SweepDomain> doms(n);
+  // domains solved by the resident kernel, and by the list sweeps
+  std::vector<qesb_handle *> res;
+  std::vector<int> res_of, str_of;  // batch indices
+  unsigned long long room = kResMarks;
+  std::vector<char> is_res(n, 0);
+  for (int i = 0; i < n; ++i) is_res[i] = res_may(h0, hs[i], itermax, &room);
+  is_res = res_choose(h0, hs, n, is_res);
+  for (int i = 0; i < n; ++i) {
+    if (is_res[i]) {
+      res.push_back(hs[i]);
+      res_of.push_back(i);
+    } else {
+      str_of.push_back(i);
+    }
+  }
+  std::vector<SweepDomain> doms;
   double cells = 0;
   std::vector<SweepDomain> pre, start;
   std::vector<int> pre_of, start_of;  // batch index of each pre-phase / start-stage domain
@@ -2509,6 +2994,11 @@ qesb_status qesb_solve_batch(qesb_handle *const *hs, int n, int itermax, float *
     ensure_divergence(h, s);
     CKS(wb.zero(h->d_err, sizeof(double) * nerr));
     h->last_pre_iterations = 0;
+    if (is_res[i]) {
+      CKS(res_prepare(h));
+      CKS(wb.zero(h->d_state, sizeof(SolveState)));
+      continue;
+    }
     if (pre_on) {
       SweepDomain p;
       CKS(sweep_domain_pre(h, p, s));
@@ -2526,20 +3016,32 @@ qesb_status qesb_solve_batch(qesb_handle *const *hs, int n, int itermax, float *
     k_pad_to_split<<<row_grid(G, G.Y, G.Z, G.X), 256, 0, s>>>(G, h->S, h->d_lam, h->d_lam_s);
     k_pad_to_split<<<row_grid(G, G.Y, G.Z, G.X), 256, 0, s>>>(G, h->S, h->d_R, h->d_R_s);
     CK(cudaGetLastError());
-    doms[i] = sweep_domain(h, itermax, (double)h->tol);
-    CKS(attach_tmaps(h, sv, doms[i], s));
+    doms.push_back(sweep_domain(h, itermax, (double)h->tol));
+    CKS(attach_tmaps(h, sv, doms.back(), s));
     cells += (double)G.XY * G.Z;
   }
   CKS(wb.flush());
+  int res_launches = 0;
+  float ms_res = 0;
+  unsigned long long t0_res = 0;
+  if (!res.empty()) {
+    CKS(res_enqueue(h0, res, itermax, s, &res_launches));
+    if (!doms.empty()) {  // the list sweeps reuse the events
+      CK(cudaStreamSynchronize(s));
+      CK(cudaEventElapsedTime(&ms_res, h0->evs[0], h0->evs[1]));
+    }
+  }
   SweepList &list = h0->blist;
-  if (list.cap < n) {
+  const int ns = (int)doms.size();
+  if (ns > 0 && list.cap < ns) {
     list.destroy();
-    CKS(list.create(n));
+    CKS(list.create(ns));
   }
   list.a.wait_limit = h0->opt_wait_limit;
-  k_sweep_stamp<<<1, 1, 0, s>>>(list.a.ctl);  // the latencies (ms_sor) count from here
   qesb_status qs = QESB_OK;
   int launched = 0, pre_launched = 0;
+  if (ns > 0) {
+  k_sweep_stamp<<<1, 1, 0, s>>>(list.a.ctl);  // the latencies (ms_sor) count from here
   CK(cudaEventRecord(h0->evs[0], s));
   if (!start.empty()) {
     // the start stages of the pre-phases that have one, as a list of their own
@@ -2597,22 +3099,27 @@ qesb_status qesb_solve_batch(qesb_handle *const *hs, int n, int itermax, float *
   sweep_tiles(doms, sv, true, h0->device);
   if (qs == QESB_OK) qs = list.upload(doms, sv.unit, s);
   if (qs == QESB_OK && h0->win_k > 0)  // each domain's first window starts from lambda as the loop begins
-    for (int i = 0; i < n && qs == QESB_OK; ++i)
-      qs = copy_floats(hs[i]->d_snap, hs[i]->d_lam_s, 2L * hs[i]->S.CS, s);
+    for (size_t q = 0; q < str_of.size() && qs == QESB_OK; ++q)
+      qs = copy_floats(hs[str_of[q]]->d_snap, hs[str_of[q]]->d_lam_s, 2L * hs[str_of[q]]->S.CS, s);
   if (qs == QESB_OK) {
     CK(cudaEventRecord(h0->evs[2], s));
     if (itermax > 0)
       qs = run_sweep_loop(sv, true, list.a, h0->device, s, cells, itermax, h0->opt_graph != 0, &h0->bgraph, h0->h_ctl,
-                          h0->h_ctl_dev, &launched, h0->win_k, n, h0->opt_pdl != 0);
+                          h0->h_ctl_dev, &launched, h0->win_k, ns, h0->opt_pdl != 0);
     CK(cudaEventRecord(h0->evs[3], s));
   }
-  const unsigned long long t0 = h0->h_ctl->t0;
+  }
+  const unsigned long long t0 = ns > 0 ? h0->h_ctl->t0 : 0;
   CK(cudaEventRecord(h0->ev[2], s));
-  for (int i = 0; i < n && qs == QESB_OK; ++i) {
-    qesb_handle *h = hs[i];
+  for (size_t q = 0; q < str_of.size() && qs == QESB_OK; ++q) {
+    qesb_handle *h = hs[str_of[q]];
     const DevGrid &G = h->G;
     k_split_mirror_ring<<<G.Y, 128, 0, s>>>(G, h->S, h->d_lam_s);
     k_split_to_pad<<<row_grid(G, G.Y, G.Z, G.X), 256, 0, s>>>(G, h->S, h->d_lam_s, h->d_lam);
+  }
+  for (int i = 0; i < n && qs == QESB_OK; ++i) {
+    qesb_handle *h = hs[i];
+    const DevGrid &G = h->G;
     k_correct<<<dim3(1, (G.FY + 7) / 8, G.FZ), dim3(32, 8), 0, s>>>(
         G, h->d_lam, h->d_in[1], h->d_in[3], h->d_in[5], h->d_flag, h->d_u0, h->d_v0, h->d_w0, h->d_dz, h->dx,
         h->dy, u ? u[i] : nullptr, v ? v[i] : nullptr, w ? w[i] : nullptr);
@@ -2630,10 +3137,12 @@ qesb_status qesb_solve_batch(qesb_handle *const *hs, int n, int itermax, float *
   cudaError_t se = cudaStreamSynchronize(s);
   if (qs != QESB_OK) return qs;
   if (se != cudaSuccess) return qesb_fail(QESB_ERR_CUDA, "batch: %s", cudaGetErrorString(se));
+  if (!res.empty()) CKS(res_finish(h0, res, res_of, true, &t0_res));
   float ms_all = 0, ms_pre = 0, ms_ref = 0;
   CK(cudaEventElapsedTime(&ms_all, h0->ev[0], h0->ev[3]));
   CK(cudaEventElapsedTime(&ms_pre, h0->evs[0], h0->evs[1]));
-  CK(cudaEventElapsedTime(&ms_ref, h0->evs[2], h0->evs[3]));
+  if (ns > 0) CK(cudaEventElapsedTime(&ms_ref, h0->evs[2], h0->evs[3]));
+  const unsigned long long t_begin = !res.empty() ? t0_res : t0;  // the first launch of the batch's iterations
   int nan_at = -1;
   for (int i = 0; i < n; ++i) {
     const SolveState sti = *hs[i]->h_state;
@@ -2646,13 +3155,13 @@ qesb_status qesb_solve_batch(qesb_handle *const *hs, int n, int itermax, float *
       st[i].converged = sti.converged;
       st[i].residual = itermax > 0 ? sti.residual : 1.0;
       st[i].ms_total = ms_all;
-      st[i].ms_sor = sti.t_done > t0 ? (double)(sti.t_done - t0) * 1e-6 : 0.0;
+      st[i].ms_sor = sti.t_done > t_begin ? (double)(sti.t_done - t_begin) * 1e-6 : 0.0;
       st[i].path = 1;
       st[i].sweeps_per_launch = 1;
-      st[i].launches = 2 * (launched + pre_launched) + (h0->win_k > 0 ? launched / h0->win_k : 0);
+      st[i].launches = 2 * (launched + pre_launched) + (h0->win_k > 0 ? launched / h0->win_k : 0) + res_launches;
       st[i].pre_iterations = hs[i]->last_pre_iterations;
       st[i].window_drift = h0->win_k > 0 && st[i].iterations >= h0->win_k ? sti.wdrift : -1.0;
-      st[i].ms_sweeps = (double)ms_pre + (double)ms_ref;
+      st[i].ms_sweeps = (double)ms_pre + (double)ms_ref + (double)ms_res;
     }
   }
   if (nan_at >= 0) return qesb_fail(QESB_ERR_NUMERIC, "NaN in lambda of batch domain %d", nan_at);

@@ -1,0 +1,126 @@
+"""Solves with lambda resident in shared memory (the default for domains that
+fit) against the oracle: grids at the edges of the tiling (one cell, one row or
+one plane per tile, ragged rows, one CTA and many), every stop, and batches
+whose domains run on groups of CTAs of different sizes. Equal bits everywhere."""
+import numpy as np
+import pytest
+
+import qesb
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+# the smallest grid; single updated rows, planes and columns; rows of one and of many 4-cell groups; sizes off
+# every multiple; long x, long y, tall; one that needs every SM
+GRIDS = [(3, 3, 2), (3, 40, 5), (40, 3, 9), (9, 7, 2), (10, 9, 3), (17, 12, 4), (47, 41, 20), (64, 33, 17),
+         (257, 40, 21), (33, 200, 12), (8, 9, 90), (130, 131, 33), (514, 30, 9), (200, 180, 60)]
+
+
+def _city(nx, ny, nz, seed=5):
+    d = qesb.Domain(nx, ny, nz, 2.0, 2.0, 1.0, qesb.city_dz(nz, 1.0, 1.03))
+    if min(nx, ny) < 30:  # no room for the generator's margins: one block in the middle
+        b = [qesb.Building(2.0 * (nx // 3), 2.0 * (ny // 3), max(2.0, 2.0 * (nx // 4)), max(2.0, 2.0 * (ny // 4)),
+                           max(1.0, nz / 3.0), 0.0)]
+        return qesb.city_build(d, b, qesb.Inflow(4.0, 10.0, 0.2, 250.0))
+    c = qesb.city_random(d, seed, 12, fp=(6, 20), h=(4, 20))
+    return qesb.city_build(d, c.buildings, c.inflow)
+
+
+def _check_winds(w, L):
+    for name, x in zip("uvw", O.correct(w.domain, w, L)):
+        np.testing.assert_array_equal(getattr(w, name), x, err_msg=name)
+
+
+@pytest.mark.parametrize("grid", GRIDS)
+def test_fixed_count_from_a_rough_start(grid):
+    """A random start (its ground plane not the mirror of plane 1), a count
+    that ends the loop: lambda, winds and every iteration's FP64 maximum."""
+    w = _city(*grid)
+    d = w.domain
+    lam0 = np.random.default_rng(3).standard_normal(d.numCellCentered()).astype(np.float32)
+    n = 11
+    with qesb.Solver_B200(d, 1e-9) as s:
+        s.lambda_ = lam0
+        st = s.solve(w, n)
+        lam, hist = s.lambda_, s.residual_history(n)
+    L, it, _, ho = O.sor(d, w, O.divergence(d, w), 1e-9, n, lam=lam0, hist=True)
+    assert st["iterations"] == it
+    np.testing.assert_array_equal(lam, L)
+    np.testing.assert_array_equal(hist[:it], ho[:it])
+    assert st["residual"] == ho[it - 1]
+    _check_winds(w, L)
+
+
+@pytest.mark.parametrize("grid", [(10, 9, 3), (47, 41, 20), (130, 61, 33)])
+@pytest.mark.parametrize("start", [None, (1.7, 5)])
+def test_phases_and_window_rule(grid, start):
+    """Start stage, pre-phase to its tolerance and reference loop to the window
+    rule, then a second solve from the kept lambda, against the oracle's chain."""
+    w = _city(*grid)
+    d = w.domain
+    R = O.divergence(d, w)
+    K, wtol, pre = 8, 5e-3, (1.85, 2e-3, 3000)
+    L = None
+    with qesb.Solver_B200(d, 1e-9) as s:
+        s.set_prephase(*pre)
+        s.set_window_rule(K, wtol)
+        if start:
+            s.set_prephase_start(*start)
+        for _ in range(2):
+            st = s.solve(w, 4000)
+            ns = 0
+            if start:
+                L, ns, *_ = O.sor(d, w, R, -1.0, start[1], omega=start[0], lam=L)
+            L, npre, *_ = O.sor(d, w, R, pre[1], pre[2], omega=pre[0], lam=L)
+            L, it, stop, drift = O.sor_window(d, w, R, 1e-9, 4000, K, wtol, lam=L)
+            assert (st["pre_iterations"], st["iterations"], st["converged"]) == (ns + npre, it, stop)
+            assert st["window_drift"] == drift
+            np.testing.assert_array_equal(s.lambda_, L)
+            _check_winds(w, L)
+
+
+@pytest.mark.parametrize("tol", [0.3, 0.05, 2e-3])
+def test_stop_on_the_iteration_of_the_rule(tol):
+    w = _city(90, 75, 24)
+    d = w.domain
+    with qesb.Solver_B200(d, tol) as s:
+        st = s.solve(w, 5000)
+        lam = s.lambda_
+    L, it, *_ = O.sor(d, w, O.divergence(d, w), tol, 5000)
+    assert (st["iterations"], st["converged"]) == (it, 1)
+    np.testing.assert_array_equal(lam, L)
+
+
+def test_batch_of_uneven_domains_and_group_sizes():
+    """Small domains that share a launch, larger ones, and one too large for
+    the chip (list sweeps), in one call: each its own oracle result."""
+    grids = [(40, 33, 9), (200, 180, 60), (64, 48, 20), (31, 77, 15), (96, 90, 40), (12, 9, 4), (640, 512, 30)]
+    ws = [_city(*g, seed=7 + i) for i, g in enumerate(grids)]
+    solvers = [qesb.Solver_B200(w.domain, 2e-2) for w in ws]
+    try:
+        for s, w in zip(solvers, ws):
+            s.set_inputs(w)
+        st = qesb.solve_batch(solvers, 60)
+        lams = [s.lambda_ for s in solvers]
+    finally:
+        for s in solvers:
+            s.close()
+    for w, x, lam in zip(ws, st, lams):
+        L, it, *_ = O.sor(w.domain, w, O.divergence(w.domain, w), 2e-2, 60)
+        assert x["iterations"] == it
+        np.testing.assert_array_equal(lam, L)
+
+
+def test_group_wait_that_runs_out_is_an_error_and_the_handle_recovers():
+    w = _city(130, 131, 33)
+    d = w.domain
+    with qesb.Solver_B200(d, 1e-9) as s:
+        s.set_option("wait_limit", 1)
+        with pytest.raises(qesb.QesbError, match="gave up"):
+            s.solve(w, 50)
+        s.set_option("wait_limit", 0)
+        s.resetLambda()
+        s.solve(w, 20)
+        lam = s.lambda_
+    L, *_ = O.sor(d, w, O.divergence(d, w), 1e-9, 20)
+    np.testing.assert_array_equal(lam, L)
