@@ -26,6 +26,12 @@ qesb_status qesb_city_walls_dev(int Nx, int Ny, int Nz, float dx, const float *d
 qesb_status qesb_conv3d_head(const void *x1, int c1, int items, int D, int H, int W, const void *Bm, int Kp, int N,
                              float *y0, const float *bias, int relu, int *err, void *stream);
 
+// The tiles (nty x ntz, at most tym rows x tzm planes) of a resident solve of an
+// X x Y x Z cell grid on this device (*nty = 0: it does not fit), the CTAs'
+// count, their threads and the floats of shared memory each takes.
+void qesb_res_tiles(int X, int Y, int Z, int device, int *nty, int *ntz, int *tym, int *tzm, int *ctas, int *threads,
+                    int *smem_floats);
+
 // A small transfer run as a kernel on `stream` (no copy engine): dst and src
 // device memory or the device alias of mapped pinned host memory, bytes a
 // multiple of 4. The caller waits for the stream before reading dst.

@@ -860,6 +860,8 @@ struct qesb_handle {
   float *d_R = nullptr;                       // padded R
   uint8_t *d_mask = nullptr;                  // padded wall mask
   float *d_pc[6] = {};                        // padded coefficients (full path)
+  float *d_cs = nullptr;                      // [7][2][CS] split coefficients and omega / sum (resident full path)
+  bool cs_ready = false;                      // d_cs holds the current inputs'
   float *d_in[6] = {};                        // natural coefficients (owned copy, or caller's)
   int *d_flag = nullptr;
   float *d_u0 = nullptr, *d_v0 = nullptr, *d_w0 = nullptr;
@@ -1084,6 +1086,42 @@ qesb_status ensure_padded_coefs(qesb_handle *h)
   return QESB_OK;
 }
 
+// The coefficients in the split layout, and omega / (their sum) (the division
+// of every update, Solver_CPU_RB.cpp:118, done once).
+__global__ void k_split_coefs(DevGrid G, SplitGeom S, const float *__restrict__ e, const float *__restrict__ f,
+                              const float *__restrict__ g, const float *__restrict__ h, const float *__restrict__ m,
+                              const float *__restrict__ n, float *__restrict__ out)
+{
+  const int j = blockIdx.y, k = blockIdx.z;
+  const long cs = 2 * S.CS;
+  for (int i = threadIdx.x + blockIdx.x * blockDim.x; i < G.X; i += gridDim.x * blockDim.x) {
+    const long c = G.cell(i, j, k), d = ((i + j + k) & 1) * S.CS + S.row(j, k, G.Y) + (i >> 1);
+    const float ve = e[c], vf = f[c], vg = g[c], vh = h[c], vm = m[c], vn = n[c];
+    out[d] = ve;
+    out[d + cs] = vf;
+    out[d + 2 * cs] = vg;
+    out[d + 3 * cs] = vh;
+    out[d + 4 * cs] = vm;
+    out[d + 5 * cs] = vn;
+    out[d + 6 * cs] = kOmega / (ve + vf + vg + vh + vm + vn);
+  }
+}
+
+qesb_status ensure_split_coefs(qesb_handle *h)
+{
+  if (h->cs_ready) return QESB_OK;
+  const DevGrid &G = h->G;
+  if (!h->d_cs) CKS(dalloc(&h->d_cs, 14 * (size_t)h->S.CS));
+  k_split_coefs<<<row_grid(G, G.Y, G.Z, G.X), 256, 0, h->stream>>>(G, h->S, h->d_in[0], h->d_in[1], h->d_in[2], h->d_in[3],
+                                                                  h->d_in[4], h->d_in[5], h->d_cs);
+  CK(cudaGetLastError());
+  h->cs_ready = true;
+  return QESB_OK;
+}
+
+const ResPlan &res_plan_of(qesb_handle *lead, const DevGrid &G, int ctas);
+int res_ctas(int device);
+
 // R for a solve: the R already computed from the same inputs (a warm start
 // computes it first), ordered after its computation, or a new one.
 void ensure_divergence(qesb_handle *h, cudaStream_t s)
@@ -1124,7 +1162,8 @@ qesb_status prepare_coefs(qesb_handle *h)
   // one the packed path is tested against) gets its padded copies here when
   // it is the only path, else at its first use.
   h->pc_ready = false;
-  if (!h->packed) CKS(ensure_padded_coefs(h));
+  h->cs_ready = false;
+  if (!h->packed) CKS(res_plan_of(h, G, res_ctas(h->device)).nty > 0 ? ensure_split_coefs(h) : ensure_padded_coefs(h));
   return QESB_OK;
 }
 
@@ -2033,8 +2072,9 @@ qesb_status res_prepare(qesb_handle *h)
 // Solves the handles' domains (R computed, err and state zeroed on s) from their current lambda to the end of their reference loops:
 // one cooperative launch per group size. Enqueues everything on s, the final
 // states' copies to the mapped buffers included; the caller waits and then
-// calls res_finish. *launches: kernels launched.
-qesb_status res_enqueue(qesb_handle *lead, const std::vector<qesb_handle *> &hs, int itermax, cudaStream_t s,
+// calls res_finish. full: with each cell's own coefficients (d_cs), the
+// reference loop alone. *launches: kernels launched.
+qesb_status res_enqueue(qesb_handle *lead, const std::vector<qesb_handle *> &hs, bool full, int itermax, cudaStream_t s,
                         int *launches)
 {
   const int n = (int)hs.size(), sms = res_ctas(lead->device);
@@ -2115,11 +2155,12 @@ qesb_status res_enqueue(qesb_handle *lead, const std::vector<qesb_handle *> &hs,
       for (int c = 0; c < 2; ++c) d.walls[c] = reinterpret_cast<uint2 *>(h->d_pc[c]);
       h->pc_ready = false;
       SweepDomain sd;
-      if (start_on(h)) {
+      if (full) d.co = h->d_cs;
+      if (start_on(h) && !full) {
         CKS(sweep_domain_start(h, sd, s));
         d.ph[d.nph++] = {sd.inv, h->d_rerr + h->pre_iters, h->d_rstate + 1, sd.tol, sd.c1, sd.itermax, 0};
       }
-      if (prephase_on(h)) {
+      if (prephase_on(h) && !full) {
         CKS(sweep_domain_pre(h, sd, s));
         d.ph[d.nph++] = {sd.inv, h->d_rerr, h->d_rstate, sd.tol, sd.c1, sd.itermax, 0};
       }
@@ -2148,7 +2189,7 @@ qesb_status res_enqueue(qesb_handle *lead, const std::vector<qesb_handle *> &hs,
     a.xstride = xstride[q];
     a.wait_limit = lead->opt_wait_limit;
     a.smem_floats = kResSmemBytes / 4;
-    CK(res_launch(a, ls[q].groups, kResThreads, s));
+    CK(res_launch(a, full, ls[q].groups, kResThreads, s));
   }
   CK(cudaEventRecord(lead->evs[1], s));
   for (size_t l = 0; l < ls.size(); ++l)
@@ -2188,13 +2229,14 @@ qesb_status res_finish(qesb_handle *lead, const std::vector<qesb_handle *> &hs, 
 }
 
 // One solve on the resident kernel: as run_iterations_sweep, in one launch.
-qesb_status run_iterations_resident(qesb_handle *h, int itermax)
+qesb_status run_iterations_resident(qesb_handle *h, bool full, int itermax)
 {
   cudaStream_t s = h->stream;
   CKS(res_prepare(h));
-  CKS(res_enqueue(h, {h}, itermax, s, &h->last_launches));
+  if (full) CKS(ensure_split_coefs(h));
+  CKS(res_enqueue(h, {h}, full, itermax, s, &h->last_launches));
   for (int q = 2; q < 4; ++q) CK(cudaEventRecord(h->evs[q], s));  // one launch runs every phase: evs[0..1]
-  h->sweeps_timed = true;
+  h->sweeps_timed = !full;
   return QESB_OK;
 }
 
@@ -2230,21 +2272,21 @@ qesb_status solve_impl(qesb_handle *h, int itermax, float *u, float *v, float *w
   CK(cudaEventRecord(h->ev[1], s));
   const bool packed = h->packed && h->opt_path == 1;
   unsigned long long room = kResMarks;
-  const bool resident = packed && res_may(h, h, itermax, &room);
+  const bool resident = res_may(h, h, itermax, &room);
   if (packed && !resident && h->opt_autotune && h->opt_variant < 0 && tuned_variant(G) < 0) {
     CKS(qesb_autotune(h, nullptr, nullptr, 0));
     CK(cudaEventRecord(h->ev[1], s));
   }
   int vi = packed ? pick_variant(h) : -1;
   // the fused tiled kernels have no window checks and no pre-phase: either runs on the sweep kernels
-  if (packed && (h->win_k > 0 || prephase_on(h)) && vi < kSplitVariant) vi = kSplitVariant + kDefaultSweep;
+  if (packed && !resident && (h->win_k > 0 || prephase_on(h)) && vi < kSplitVariant) vi = kSplitVariant + kDefaultSweep;
   const bool split = packed && vi >= kSplitVariant;
   const Variant *var = packed && !split && !resident ? &kVariants[vi] : nullptr;
   h->last_launches = 0;
   h->last_pre_iterations = 0;
   h->sweeps_timed = false;
   if (itermax > 0) {
-    if (resident) CKS(run_iterations_resident(h, itermax));
+    if (resident) CKS(run_iterations_resident(h, !packed, itermax));
     else if (split) CKS(run_iterations_sweep(h, kSweepVariants[vi - kSplitVariant], itermax));
     else if (var) CKS(run_iterations_tiled(h, *var, itermax));
     else CKS(run_iterations_full(h, itermax));
@@ -2275,7 +2317,7 @@ qesb_status solve_impl(qesb_handle *h, int itermax, float *u, float *v, float *w
     st->ms_sor = b;
     st->path = packed ? 1 : 0;
     st->sweeps_per_launch = var ? var->K : 1;
-    st->launches = 2 + (packed ? h->last_launches : 4 * st->iterations);
+    st->launches = 2 + (packed || resident ? h->last_launches : 4 * st->iterations);
     st->pre_iterations = h->last_pre_iterations;
     st->window_drift = h->win_k > 0 && st->iterations >= h->win_k ? h->h_state->wdrift : -1.0;
     st->ms_sweeps = -1.0;
@@ -2322,7 +2364,7 @@ void free_all(qesb_handle *h)
                   h->d_own_in[2], h->d_own_in[3], h->d_own_in[4], h->d_own_in[5], h->d_own_flag,
                   h->d_own_u0, h->d_own_v0, h->d_own_w0, h->d_dz, h->d_vmax, h->d_inv, h->d_val,
                   h->d_inv_pre, h->d_inv_start, h->d_bad, h->d_err, h->d_state, h->d_u, h->d_v, h->d_w, h->d_wbits,
-                  h->d_wcut, h->d_snap, h->d_tmaps, h->d_rerr, h->rlist.blk, h->rlist.xbuf};
+                  h->d_wcut, h->d_snap, h->d_tmaps, h->d_rerr, h->d_cs, h->rlist.blk, h->rlist.xbuf};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   h->list.destroy();
@@ -3025,7 +3067,7 @@ qesb_status qesb_solve_batch(qesb_handle *const *hs, int n, int itermax, float *
   float ms_res = 0;
   unsigned long long t0_res = 0;
   if (!res.empty()) {
-    CKS(res_enqueue(h0, res, itermax, s, &res_launches));
+    CKS(res_enqueue(h0, res, false, itermax, s, &res_launches));
     if (!doms.empty()) {  // the list sweeps reuse the events
       CK(cudaStreamSynchronize(s));
       CK(cudaEventElapsedTime(&ms_res, h0->evs[0], h0->evs[1]));
@@ -3191,6 +3233,23 @@ qesb_status qesb_set_prephase(qesb_handle *h, float omega, float tol, int max_it
 }
 
 }  // extern "C"
+
+void qesb_res_tiles(int X, int Y, int Z, int device, int *nty, int *ntz, int *tym, int *tzm, int *ctas, int *threads,
+                    int *smem_floats)
+{
+  DevGrid G{};
+  G.X = X;
+  G.Y = Y;
+  G.Z = Z;
+  *ctas = res_ctas(device);
+  const ResPlan p = res_plan(G, *ctas);
+  *nty = p.nty;
+  *ntz = p.ntz;
+  *tym = p.tym;
+  *tzm = p.tzm;
+  *threads = kResThreads;
+  *smem_floats = kResSmemBytes / 4;
+}
 
 qesb_status qesb_handle_grid(qesb_handle *h, int *Nx, int *Ny, int *Nz, int *device)
 {

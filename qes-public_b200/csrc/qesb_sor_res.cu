@@ -38,6 +38,11 @@
 // out of L2 per CTA and the wait for the slowest neighbour. Small domains are all
 // latency: two exchanges of about 1.2 us each.
 //
+// FULL: every cell has its own six coefficients (no wall mask): they stream from
+// L2, 28 B a cell with omega / (their sum), while lambda still stays here. An
+// iteration of 151 x 133 x 61 takes 12 us, with the four launches of the
+// streaming loop (both colours, mirror, poll; 68 B a cell) 33.
+//
 // The arithmetic is the other sweeps' (Solver_CPU_RB.cpp:118-125, the same
 // operation order), so results are bit-identical. The ground mirror
 // lambda(k=0) <- lambda(k=1) of every iteration (Solver_CPU_RB.cpp:155-162)
@@ -138,6 +143,7 @@ struct ResTile {
   float *lam;
   const float *R;
   const uint8_t *mask;
+  const float *co;  // full coefficients, or null
   __device__ __forceinline__ long gidx(int c, int k, int j, int q4) const
   {
     return c * CS + ((long)(k0 + k) * Y + (j0 + j)) * PQ + 4 * q4;
@@ -186,6 +192,22 @@ __device__ __forceinline__ float res_pick(uint32_t m, float a, float v)
   return __uint_as_float((__float_as_uint(a) & k) | (__float_as_uint(v) & ~k));
 }
 
+// The same with each cell's own coefficients: at q = 0 .. 6 the split arrays of e f g h m n and omega / (their sum)
+// lie cs floats apart.
+template <int I0>
+__device__ __forceinline__ float4 res_row_full(const float *q, long cs, float c1, float4 C, float edge, float4 N, float4 S,
+                                               float4 T, float4 B, float4 O, float4 R)
+{
+  auto ld = [&](int i) { return __ldg(reinterpret_cast<const float4 *>(q + i * cs)); };
+  const float4 e = ld(0), f = ld(1), g = ld(2), h = ld(3), m = ld(4), n = ld(5), v = ld(6);
+  const float x0 = I0 ? C.x : edge, x1 = I0 ? C.y : C.x, x2 = I0 ? C.z : C.y, x3 = I0 ? C.w : C.z, x4 = I0 ? edge : C.w;
+  return make_float4(
+      v.x * (e.x * x1 + f.x * x0 + g.x * N.x + h.x * S.x + m.x * T.x + n.x * B.x - R.x) + c1 * O.x,
+      v.y * (e.y * x2 + f.y * x1 + g.y * N.y + h.y * S.y + m.y * T.y + n.y * B.y - R.y) + c1 * O.y,
+      v.z * (e.z * x3 + f.z * x2 + g.z * N.z + h.z * S.z + m.z * T.z + n.z * B.z - R.z) + c1 * O.z,
+      v.w * (e.w * x4 + f.w * x3 + g.w * N.w + h.w * S.w + m.w * T.w + n.w * B.w - R.w) + c1 * O.w);
+}
+
 __device__ __forceinline__ void res_exact(ResMax &mx, float a, float b)
 {
   const double y = fabs((double)a - (double)b);
@@ -203,6 +225,7 @@ __device__ __forceinline__ bool res_reaches(ResMax &mx, float d)
 }
 
 // One task: the lanes' columns of colour c over a run of rows. xb: this CTA's exchange slots of colour c.
+template <bool FULL>
 __device__ __forceinline__ void res_task(const ResTile &t, const short *segs, int task, int c, ulonglong2 *xb,
                                          unsigned mark, ResMax &mx)
 {
@@ -224,8 +247,17 @@ __device__ __forceinline__ void res_task(const ResTile &t, const short *segs, in
   const int kd = 4 * t.nq4;
   int rx = t.rs + (rrow - c * (t.tz - t.rp) * t.ty) * P + 16 * q4;  // R in shared memory: [2][rp][ty][P]
   const float *gR = t.R + t.gidx(c, k, ja, q4);
-  ResCoef K = sm<ResCoef>(t.cf + 32 * k);
-  if (k == 0 && t.base0 == 31u) K.n = 0.0f;
+  ResCoef K;
+  const float *gC = nullptr;
+  long cs = 0;
+  if (FULL) {
+    gC = t.co + t.gidx(c, k, ja, q4);
+    cs = 2 * t.CS;
+    K.c1 = sm<float>(t.cf + 28);
+  } else {
+    K = sm<ResCoef>(t.cf + 32 * k);
+    if (k == 0 && t.base0 == 31u) K.n = 0.0f;
+  }
   const bool ground = ok && t.k0 == 1 && k == 0;
   const bool pB = ok && t.pubB && k == 0, pT = ok && t.pubT && k == t.tz - 1;
   const bool anyp = __any_sync(0xffffffffu, pB || pT), split = t.split;
@@ -240,7 +272,7 @@ __device__ __forceinline__ void res_task(const ResTile &t, const short *segs, in
     if (j == jS && ok) res_publish(xb + 2 * (k * t.nq4 + q4), mark, V);
     if (j == jN && ok) res_publish(xb + 2 * ((t.tzm + k) * t.nq4 + q4), mark, V);
   };
-  auto update = [&](auto tag, float4 C_, float4 N_, float4 S_, int o_, float4 R_, uint32_t km, float4 &O_) {
+  auto update = [&](auto tag, float4 C_, float4 N_, float4 S_, int o_, float4 R_, uint32_t km, float4 &O_, int dc = 0) {
     constexpr int I0 = decltype(tag)::v;
     const float4 T = lds4(o_ + dx + PS), B = lds4(o_ + dx - PS);
     O_ = lds4(o_);
@@ -250,7 +282,8 @@ __device__ __forceinline__ void res_task(const ResTile &t, const short *segs, in
       const float e = sm<float>(o_ + dx + (I0 ? 16 : -4));
       edge = lane == (I0 ? 31 : 0) ? e : edge;
     }
-    float4 V = res_row<I0>(K, C_, edge, N_, S_, T, B, O_, R_);
+    float4 V = FULL ? res_row_full<I0>(gC + dc, cs, K.c1, C_, edge, N_, S_, T, B, O_, R_)
+                    : res_row<I0>(K, C_, edge, N_, S_, T, B, O_, R_);
     V.x = res_pick<0>(km, O_.x, V.x);
     V.y = res_pick<1>(km, O_.y, V.y);
     V.z = res_pick<2>(km, O_.z, V.z);
@@ -279,7 +312,7 @@ __device__ __forceinline__ void res_task(const ResTile &t, const short *segs, in
     const uint32_t k0 = sm<uint32_t>(ko) | out, k1 = sm<uint32_t>(ko + kd) | out;
     float4 O0, O1;
     const float4 V0 = update(ResPar<I0>{}, C, N0, S, o, R0, k0, O0);
-    const float4 V1 = update(ResPar<1 - I0>{}, N0, N1, C, o + P, R1, k1, O1);
+    const float4 V1 = update(ResPar<1 - I0>{}, N0, N1, C, o + P, R1, k1, O1, PQ);
     if (ok) {
       sts4(o, V0);
       sts4(o + P, V1);
@@ -299,6 +332,7 @@ __device__ __forceinline__ void res_task(const ResTile &t, const short *segs, in
     o += 2 * P;
     rx += 2 * P;
     ko += 2 * kd;
+    if (FULL) gC += 2 * PQ;
   };
   auto row1 = [&](int j, auto tag) {
     constexpr int I0 = decltype(tag)::v;
@@ -349,6 +383,7 @@ __device__ __forceinline__ void res_wall(const ResTile &t, uint2 w, bool on, int
   if (res_reaches(mx, fabsf(nv - ov))) res_exact(mx, nv, ov);
 }
 
+template <bool FULL>
 __global__ void __launch_bounds__(kResMaxThreads, 1) k_sor_res(ResArgs a)
 {
   __shared__ unsigned long long s_err[2];  // CTA's exact max|dlambda| (double bits), by iteration parity
@@ -407,6 +442,7 @@ __global__ void __launch_bounds__(kResMaxThreads, 1) k_sor_res(ResArgs a)
       t.lam = D.lam;
       t.R = D.R;
       t.mask = D.mask;
+      t.co = D.co;
       const int jt = rank % nty, kt = rank / nty;
       t.j0 = 1 + (int)((long)(D.Y - 2) * jt / nty);
       t.ty = 1 + (int)((long)(D.Y - 2) * (jt + 1) / nty) - t.j0;
@@ -541,7 +577,7 @@ __global__ void __launch_bounds__(kResMaxThreads, 1) k_sor_res(ResArgs a)
     // the ground is solid (counted on one row: either choice gives the same results).
     {
       int open = 0, closed = 0;
-      if (t.k0 == 1)
+      if (!FULL && t.k0 == 1)
         for (int q = tid; q < t.X / 2; q += NT) {
           const unsigned m = __ldg(t.mask + t.gidx(0, 0, t.ty / 2, 0) + q);
           open += m == 63u;
@@ -567,7 +603,7 @@ __global__ void __launch_bounds__(kResMaxThreads, 1) k_sor_res(ResArgs a)
         const long g = t.gidx(c, k, j, q4);
         const float4 R = __ldg(reinterpret_cast<const float4 *>(t.R + g));
         if (k < t.rp) sts4(t.rs + c * t.rp * t.ty * t.P + 16 * i, R);
-        const uint32_t m = __ldg(reinterpret_cast<const uint32_t *>(t.mask + g));
+        const uint32_t m = FULL ? 0x3f3f3f3fu : __ldg(reinterpret_cast<const uint32_t *>(t.mask + g));
         const float rv[4] = {R.x, R.y, R.z, R.w};
         const int I0 = (c + t.j0 + j + t.k0 + k) & 1;
         uint32_t keep = 0;
@@ -577,7 +613,7 @@ __global__ void __launch_bounds__(kResMaxThreads, 1) k_sor_res(ResArgs a)
           const unsigned mu = (m >> (8 * u)) & 63u;
           if (x < 1 || x > t.X - 2) {
             keep |= 0xffu << (8 * u);
-          } else if (mu != (k == 0 ? t.base0 : 63u)) {
+          } else if (!FULL && mu != (k == 0 ? t.base0 : 63u)) {
             keep |= 0xffu << (8 * u);
             const int at = atomicAdd(&s_nw[c], 1);
             const uint2 w = make_uint2((unsigned)(t.at(c, k, j, q4) / 4 + u) | mu << 16 | (unsigned)k << 22, __float_as_uint(rv[u]));
@@ -598,6 +634,12 @@ __global__ void __launch_bounds__(kResMaxThreads, 1) k_sor_res(ResArgs a)
         if (!res_wait(&sy->bar, s_target, limit, a.ctl)) s_bad = 1;
       }
     };
+    if (D.alias) {
+      __syncthreads();
+      if (tid == 0) meet();
+      __syncthreads();
+      if (s_bad) return;
+    }
     unsigned iters = 0;  // iterations of all phases
     bool dead = false;
     for (int ph = 0; ph < D.nph && !dead; ++ph) {
@@ -607,10 +649,11 @@ __global__ void __launch_bounds__(kResMaxThreads, 1) k_sor_res(ResArgs a)
         s_thr[0] = s_thr[1] = 0;
       }
       __syncthreads();
-      for (int i = tid; i < t.tz * 64; i += NT) sm<float>(t.inv + 4 * i) = __ldg(F.inv + (long)t.k0 * 64 + i);
+      for (int i = tid; !FULL && i < t.tz * 64; i += NT) sm<float>(t.inv + 4 * i) = __ldg(F.inv + (long)t.k0 * 64 + i);
       for (int i = tid; i < t.tz * 8; i += NT) {
         const int k = t.k0 + (i >> 3), q = i & 7;
-        sm<float>(t.cf + 4 * i) = q < 6 ? __ldg(D.val + q * t.Z + k)
+        if (FULL) sm<float>(t.cf + 4 * i) = F.c1;
+        else sm<float>(t.cf + 4 * i) = q < 6 ? __ldg(D.val + q * t.Z + k)
                                         : (q == 6 ? __ldg(F.inv + (long)k * 64 + (i < 8 ? t.base0 : 63u)) : F.c1);
       }
       __syncthreads();
@@ -667,7 +710,7 @@ __global__ void __launch_bounds__(kResMaxThreads, 1) k_sor_res(ResArgs a)
             }
           }
           ulonglong2 *xb = slots(c, rank);
-          if (s_nw[c]) {
+          if (!FULL && s_nw[c]) {
             for (int b = warp * 32; b < s_nw[c]; b += NT) {
               const int i = b + lane;
               const bool on = i < s_nw[c];
@@ -678,7 +721,7 @@ __global__ void __launch_bounds__(kResMaxThreads, 1) k_sor_res(ResArgs a)
             __syncthreads();
           }
           for (int task = warp; task < t.ntask; task += NW) {
-            res_task(t, s_seg, task, c, xb, mark, mx);
+            res_task<FULL>(t, s_seg, task, c, xb, mark, mx);
             if (lane == 0) atomicMax(&s_thr[par], __float_as_uint(mx.thr));
             mx.thr = fmaxf(mx.thr, __uint_as_float(*reinterpret_cast<volatile unsigned *>(&s_thr[par])));
           }
@@ -779,14 +822,15 @@ __global__ void __launch_bounds__(kResMaxThreads, 1) k_sor_res(ResArgs a)
   }
 }
 
-cudaError_t res_launch(const ResArgs &a, int groups, int threads, cudaStream_t s)
+cudaError_t res_launch(const ResArgs &a, bool full, int groups, int threads, cudaStream_t s)
 {
   const size_t smem = sizeof(float) * (size_t)a.smem_floats;
-  cudaError_t e = cudaFuncSetAttribute(k_sor_res, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  void (*const fn)(ResArgs) = full ? k_sor_res<true> : k_sor_res<false>;
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   ResArgs b = a;
   void *args[] = {&b};
-  return cudaLaunchCooperativeKernel((const void *)k_sor_res, dim3(groups * a.gsz), dim3(threads), args, smem, s);
+  return cudaLaunchCooperativeKernel((const void *)fn, dim3(groups * a.gsz), dim3(threads), args, smem, s);
 }
 
 }  // namespace qesb

@@ -42,12 +42,14 @@ struct ResDomain {
   const float *R;
   const uint8_t *mask;
   const float *val;  // [6][Z]
+  const float *co;   // full coefficients instead of mask and val: [7][2][CS] e f g h m n, omega / (their sum)
   float *snap;       // [2][CS] window snapshot
   uint2 *walls[2];   // [(Y - 2) (Z - 2) 4 nq4] room for each colour's wall cells
   double wtol;
   int nph;
   ResPhase ph[kResPhases];
   ResSync *sync;
+  bool alias;        // lam lies in the exchange buffer (the start is read by all CTAs before the first publishes)
 };
 
 struct ResCtl {
@@ -69,7 +71,7 @@ struct ResArgs {
 };
 
 // Launches the kernel (cooperatively: its CTAs wait on one another) with
-// groups * a.gsz CTAs of `threads` threads on s.
-cudaError_t res_launch(const ResArgs &a, int groups, int threads, cudaStream_t s);
+// groups * a.gsz CTAs of `threads` threads on s; full: the domains bring their own coefficients (co).
+cudaError_t res_launch(const ResArgs &a, bool full, int groups, int threads, cudaStream_t s);
 
 }  // namespace qesb

@@ -124,3 +124,53 @@ def test_group_wait_that_runs_out_is_an_error_and_the_handle_recovers():
         lam = s.lambda_
     L, *_ = O.sor(d, w, O.divergence(d, w), 1e-9, 20)
     np.testing.assert_array_equal(lam, L)
+
+
+def _cut(w, seed=4):
+    """Arbitrary face coefficients beside the walls and in one cell of twenty."""
+    d = w.domain
+    rng = np.random.default_rng(seed)
+    near = (w.e == 0) | (w.g == 0) | (w.m == 0) | (rng.random(w.e.size) < 0.05)
+    for name in w.FIELDS_CELL:
+        a = getattr(w, name)
+        a[near] *= (0.1 + 0.9 * rng.random(near.sum())).astype(np.float32)
+        a[near & (a == 0)] = np.float32(1e-3)  # no cell without an open face
+    assert d.numCellCentered() == w.e.size
+    return w
+
+
+@pytest.mark.parametrize("grid", [(3, 3, 2), (9, 7, 2), (17, 12, 4), (47, 41, 20), (257, 40, 21), (33, 200, 12),
+                                  (130, 131, 33)])
+def test_full_coefficients(grid):
+    """Cells with six coefficients of their own: the handle's solve (fixed
+    count from a rough start, then to the window rule) and the solve without
+    allocation, against the oracle."""
+    import torch
+
+    w = _cut(_city(*grid))
+    d = w.domain
+    R = O.divergence(d, w)
+    lam0 = np.random.default_rng(3).standard_normal(d.numCellCentered()).astype(np.float32)
+    n = 11
+    L, it, _, ho = O.sor(d, w, R, 1e-9, n, lam=lam0, hist=True)
+    with qesb.Solver_B200(d, 1e-9) as s:
+        s.set_option("path", 0)  # the smallest grid's one cell would pass for a wall mask
+        s.lambda_ = lam0
+        st = s.solve(w, n)
+        assert (st["path"], st["iterations"]) == (0, it)
+        np.testing.assert_array_equal(s.lambda_, L)
+        np.testing.assert_array_equal(s.residual_history(n)[:it], ho[:it])
+        _check_winds(w, L)
+        s.set_window_rule(8, 1e-2)
+        st = s.solve(w, 150, set_inputs=False)  # these random matrices diverge later on, in the oracle too
+        Lw, itw, stop, drift = O.sor_window(d, w, R, 1e-9, 150, 8, 1e-2, lam=L)
+        assert (st["iterations"], st["converged"], st["window_drift"]) == (itw, stop, drift)
+        np.testing.assert_array_equal(s.lambda_, Lw)
+    dev = [torch.from_numpy(a).cuda() for a in (*w.inputs(), lam0.copy())]
+    out = [torch.empty(d.numFaceCentered(), device="cuda") for _ in range(3)]
+    torch.cuda.synchronize()
+    st = qesb.solve_noalloc(d, 1e-9, n, *[t.data_ptr() for t in dev], *[t.data_ptr() for t in out])
+    assert st["iterations"] == it and st["residual"] == ho[it - 1]
+    np.testing.assert_array_equal(dev[-1].cpu().numpy(), L)
+    for name, t, x in zip("uvw", out, O.correct(d, w, L)):
+        np.testing.assert_array_equal(t.cpu().numpy(), x, err_msg=name)
