@@ -1154,8 +1154,14 @@ __global__ void __launch_bounds__(192, 1) k_conv_zflat3(const __grid_constant__ 
 
 // Weight gradient: dW[t*cin + c][n] += sum_v X[v + off(t)][c] * dY[v][n] over
 // this CTA's voxel range. M-tile = 128 rows of (t, c); K = voxels in chunks
-// of 64; both operands MN-major (channels contiguous). Partial sums from the
-// CTAs of a row tile meet in dW (FP32) by atomicAdd.
+// of 64; both operands MN-major (channels contiguous), gathered by asynchronous
+// copies two chunks ahead of the MMAs. Partial sums from the CTAs of a row tile
+// meet in dW (FP32) by atomic adds, four floats each where dW is aligned.
+// The gather bounds it (27 taps of 16 bytes a voxel and 8 channels): loads that
+// each chunk waits for, divisions for every voxel and scalar atomics took
+// 103 us for 16 -> 16 channels on 64 x 64 x 32 voxels, this form takes 53;
+// 64 + 32 -> 32 channels on 32 x 32 x 16: 161 and 45.
+constexpr int kWgStages = 3;
 template <int N>
 __global__ void __launch_bounds__(128) k_conv_wgrad(ConvIn in, ConvGeom g, const __nv_bfloat16 *__restrict__ dY,
                                                    long vchunk, float *__restrict__ dW, int *err)
@@ -1163,7 +1169,7 @@ __global__ void __launch_bounds__(128) k_conv_wgrad(ConvIn in, ConvGeom g, const
   constexpr uint32_t SA = 128 * 64 * 2, SB = N * 64 * 2, STAGE = SA + SB;
   constexpr uint32_t NCOLS = N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : 256;
   extern __shared__ __align__(1024) uint8_t sm[];
-  __shared__ __align__(8) uint64_t mbar[2];
+  __shared__ __align__(8) uint64_t mbar[kWgStages];
   __shared__ __align__(8) uint64_t mdrain;  // completion of every issued MMA, after a wait gave up
   __shared__ uint32_t tmem_base;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1174,8 +1180,8 @@ __global__ void __launch_bounds__(128) k_conv_wgrad(ConvIn in, ConvGeom g, const
   if (vb >= ve) return;
   if (warp == 0) umma::tmem_alloc(&tmem_base, NCOLS);
   if (tid == 0) {
-    umma::mbar_init(&mbar[0], 1);
-    umma::mbar_init(&mbar[1], 1);
+#pragma unroll
+    for (int q = 0; q < kWgStages; ++q) umma::mbar_init(&mbar[q], 1);
     umma::mbar_init(&mdrain, 1);
     umma::fence_mbar_init();
   }
@@ -1184,69 +1190,105 @@ __global__ void __launch_bounds__(128) k_conv_wgrad(ConvIn in, ConvGeom g, const
   umma::fence_after_sync();
   const uint32_t tmem = tmem_base;
   constexpr uint32_t idesc = umma::idesc_bf16(128, N, 1, 1);
-  // this thread: voxel column kv = tid % 64 of each chunk; row groups rg = tid/64 + 2 i
+  // this thread: voxel column kv = tid % 64 of each chunk; row groups rg = tid/64 + 2 i: their tap (packed, 2 bits
+  // an axis; -1: none) and channel
   const int kv = tid & 63;
   int tg[8], cg[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int m = mt0 + 8 * ((tid >> 6) + 2 * i);
-    tg[i] = m < Mrows ? m / cin : 27;
-    cg[i] = m < Mrows ? m - tg[i] * cin : 0;
+    const int t = m / cin;
+    tg[i] = m < Mrows ? (t / 9) << 4 | (t / 3 % 3) << 2 | t % 3 : -1;
+    cg[i] = m < Mrows ? m - t * cin : 0;
   }
   const int nk = (int)((ve - vb + 63) / 64);
-  bool ok = true;
-  for (int j = 0; j < nk && ok; ++j) {
-    const int s = j & 1;
-    if (j >= 2) ok = umma::mbar_wait(&mbar[s], ((j - 2) >> 1) & 1, kWaitLimit);
-    if (!ok) break;
-    uint8_t *sa = sm + s * STAGE, *sb = sa + SA;
-    const long v = vb + (long)j * 64 + kv;
+  // the voxel of the next chunk to be staged; it moves 64 on with each (no divisions)
+  long v = vb + kv;
+  int x = (int)(v % g.W), y = (int)((v / g.W) % g.H), z = (int)(v / ((long)g.W * g.H));
+  int zb = z - z % g.Dc;  // first plane of its item
+  auto stage = [&](int j) {
+    uint8_t *sa = sm + (j % kWgStages) * STAGE, *sb = sa + SA;
     const bool vin = v < ve;
-    const int x = vin ? (int)(v % g.W) : 0, y = vin ? (int)((v / g.W) % g.H) : 0,
-              z = vin ? (int)(v / ((long)g.W * g.H)) : 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      uint4 val = make_uint4(0, 0, 0, 0);
-      if (vin && tg[i] < 27) {
-        int dz, dy, dx;
-        tap_offset(tg[i], dz, dy, dx);
-        val = load_in8(in, g, z, z + dz, y + dy, x + dx, cg[i]);
+      const int zz = z + (tg[i] >> 4) - 1, yy = y + (tg[i] >> 2 & 3) - 1, xx = x + (tg[i] & 3) - 1, c = cg[i];
+      const bool in_ = vin && tg[i] >= 0 && zz >= zb && zz < zb + g.Dc && (unsigned)yy < (unsigned)g.H &&
+                       (unsigned)xx < (unsigned)g.W;
+      const __nv_bfloat16 *p = in.x1;
+      if (in_) {
+        if (c >= in.c1) p = in.x2 + (((long)zz * g.H + yy) * g.W + xx) * in.c2 + (c - in.c1);
+        else if (in.up1) p = in.x1 + (((long)(zz >> 1) * (g.H >> 1) + (yy >> 1)) * (g.W >> 1) + (xx >> 1)) * in.c1 + c;
+        else p = in.x1 + (((long)zz * g.H + yy) * g.W + xx) * in.c1 + c;
       }
-      *reinterpret_cast<uint4 *>(sa + off_mnmajor(8 * ((tid >> 6) + 2 * i), kv, 128)) = val;
+      cp16_zfill(sa + off_mnmajor(8 * ((tid >> 6) + 2 * i), kv, 128), p, in_);
     }
     for (int idx = tid; idx < N / 8 * 64; idx += 128) {
       const int ng = idx >> 6, k = idx & 63;
       const long vv = vb + (long)j * 64 + k;
-      uint4 val = make_uint4(0, 0, 0, 0);
-      if (vv < ve) val = __ldg(reinterpret_cast<const uint4 *>(dY + vv * N + 8 * ng));
-      *reinterpret_cast<uint4 *>(sb + off_mnmajor(8 * ng, k, N)) = val;
+      cp16_zfill(sb + off_mnmajor(8 * ng, k, N), vv < ve ? dY + vv * N + 8 * ng : dY, vv < ve);
     }
+    v += 64;
+    x += 64;
+    while (x >= g.W) {
+      x -= g.W;
+      if (++y == g.H) {
+        y = 0;
+        ++z;
+        if (z == zb + g.Dc) zb = z;
+      }
+    }
+  };
+  bool ok = true;
+  // two chunks ahead of the MMAs; one copy group per chunk (empty past the end)
+  stage(0);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  if (nk > 1) stage(1);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int j = 0; j < nk; ++j) {
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
     umma::fence_smem_async();
     __syncthreads();
     if (tid == 0) {
       umma::fence_after_sync();
-      const uint32_t a0 = umma::smem_u32(sa), b0 = umma::smem_u32(sb);
+      const uint32_t a0 = umma::smem_u32(sm + (j % kWgStages) * STAGE), b0 = a0 + SA;
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk)
         umma::mma_bf16(tmem, umma::desc(a0 + kk * 2 * 16 * 128, 16 * 128, 128),
                        umma::desc(b0 + kk * 2 * (N / 8) * 128, (N / 8) * 128, 128), idesc,
                        (j > 0 || kk > 0) ? 1u : 0u);
-      umma::mma_commit(&mbar[s]);
+      umma::mma_commit(&mbar[j % kWgStages]);
     }
+    if (j + 2 < nk) {  // into the stage that the MMA of chunk j - 1 has read
+      if (j >= 1) ok = umma::mbar_wait(&mbar[(j - 1) % kWgStages], ((j - 1) / kWgStages) & 1, kWaitLimit);
+      if (__syncthreads_or(!ok)) {
+        ok = false;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        break;
+      }
+      stage(j + 2);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  if (ok) ok = umma::mbar_wait(&mbar[(nk - 1) & 1], ((nk - 1) >> 1) & 1, kWaitLimit);
+  if (ok) ok = umma::mbar_wait(&mbar[(nk - 1) % kWgStages], ((nk - 1) / kWgStages) & 1, kWaitLimit);
   umma::fence_after_sync();
   if (!ok) {
     if (lane == 0) atomicExch(err, 1);
     umma::mma_drain(&mdrain, tid == 0, kWaitLimit);
   } else {
     const int m = mt0 + warp * 32 + lane;
+    const bool al16 = (reinterpret_cast<uintptr_t>(dW) & 15) == 0;
     for (int c0 = 0; c0 < N; c0 += 8) {
       float a[8];
       umma::tmem_ld8(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, a);
-      if (m < Mrows) {
+      if (m < Mrows && !al16) {
 #pragma unroll
         for (int q = 0; q < 8; ++q) atomicAdd(dW + (long)m * N + c0 + q, a[q]);
+      } else if (m < Mrows) {
+#pragma unroll
+        for (int q = 0; q < 8; q += 4)
+          asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dW + (long)m * N + c0 + q), "f"(a[q]),
+                       "f"(a[q + 1]), "f"(a[q + 2]), "f"(a[q + 3])
+                       : "memory");
       }
     }
   }
@@ -1626,7 +1668,7 @@ template <int N>
 qesb_status launch_wgrad(const ConvIn &in, const ConvGeom &g, const __nv_bfloat16 *dY, long vchunk, float *dW,
                          int *err, cudaStream_t s)
 {
-  constexpr int smem = 2 * (128 * 64 * 2 + N * 64 * 2);
+  constexpr int smem = kWgStages * (128 * 64 * 2 + N * 64 * 2);
   static bool attr = false;
   if (!attr) {
     cudaError_t e = cudaFuncSetAttribute(k_conv_wgrad<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

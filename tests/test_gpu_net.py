@@ -171,6 +171,37 @@ def test_conv3d_weight_gradient(D, H, W, ci, co, up):
     np.testing.assert_allclose(dW.view(27 * cin, co).cpu().double().numpy(), ref.numpy(), rtol=1e-4, atol=1e-3)
 
 
+# Rows shorter and longer than a 64-voxel chunk, ragged last chunks, one to nine
+# chunks a CTA, dW on and off a 16-byte boundary. The BF16 products are exact in
+# FP32, so the error is that of summing V of them in any order: below
+# V 2^-23 sum |x dy|.
+@pytest.mark.parametrize("off", [0, 1])
+@pytest.mark.parametrize("D,H,W,ci,co,vchunk", [(7, 9, 1, 16, 16, 64), (3, 5, 21, 16, 32, 128), (2, 3, 97, 48, 64, 576),
+                                                (1, 1, 40, 16, 16, 64), (2, 2, 48, 16, 16, 192)])
+def test_conv3d_weight_gradient_chunks(D, H, W, ci, co, vchunk, off):
+    import torch
+    torch.manual_seed(D + H + W)
+    x, dy = _bf16(torch.randn(1, ci, D, H, W)), _bf16(torch.randn(1, co, D, H, W))
+
+    def grad(a, b):
+        w = torch.zeros(co, ci, 3, 3, 3, dtype=torch.float64, requires_grad=True)
+        (torch.nn.functional.conv3d(a.double(), w, padding=1) * b.double()).sum().backward()
+        return w.grad.permute(2, 3, 4, 1, 0).reshape(27 * ci, co).numpy()
+
+    ref, tol = grad(x, dy), D * H * W * 2.0 ** -23 * grad(x.abs(), dy.abs())
+    dev = "cuda:0"
+    buf = torch.zeros(27 * ci * co + 8, dtype=torch.float32, device=dev)
+    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    xd, dyd = _cl(x).to(dev), _cl(dy).to(dev)
+    qesb.check(qesb.lib().qesb_conv3d_wgrad(xd.data_ptr(), ci, 0, None, 0, D, H, W, dyd.data_ptr(), co, vchunk,
+                                            buf.data_ptr() + 4 * off, err.data_ptr(), None))
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    out = buf.cpu().double().numpy()
+    assert np.all(np.abs(out[off:off + 27 * ci * co].reshape(27 * ci, co) - ref) <= tol)
+    assert np.all(out[:off] == 0) and np.all(out[off + 27 * ci * co:] == 0)
+
+
 # ---------------------------------------------------------------------------
 # direct conv3d kernel (rows of 128 voxels): same contract as the implicit GEMM
 # ---------------------------------------------------------------------------
