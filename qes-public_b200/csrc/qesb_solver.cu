@@ -2275,6 +2275,9 @@ qesb_status solve_impl(qesb_handle *h, int itermax, float *u, float *v, float *w
   const bool resident = res_may(h, h, itermax, &room);
   if (packed && !resident && h->opt_autotune && h->opt_variant < 0 && tuned_variant(G) < 0) {
     CKS(qesb_autotune(h, nullptr, nullptr, 0));
+    // the timed sweeps counted iterations and wrote maxima of their own
+    CK(zero_async(h->d_err, sizeof(double) * nerr, s));
+    CK(zero_async(h->d_state, sizeof(SolveState), s));
     CK(cudaEventRecord(h->ev[1], s));
   }
   int vi = packed ? pick_variant(h) : -1;

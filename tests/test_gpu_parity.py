@@ -255,6 +255,31 @@ def test_full_size_city800_bit_exact_against_oracle():
     np.testing.assert_array_equal(w.w, wo)
 
 
+@pytest.mark.parametrize("phases", [False, True])
+def test_first_solve_that_tunes_its_grid_is_exact(phases):
+    """The autotune option times sweeps inside the first solve of a grid too
+    large for shared memory; that solve's count, history, lambda and winds are
+    the oracle's all the same."""
+    d = qesb.Domain(400 + 4 * phases, 300, 50, 2.0, 2.0, 1.0, qesb.city_dz(50, 1.0, 1.03))
+    c = qesb.city_random(d, 5, 12, fp=(6, 20), h=(4, 20))
+    w = qesb.city_build(d, c.buildings, c.inflow)
+    n, n_pre = 4, 3
+    with qesb.Solver_B200(d, 1e-9) as s:
+        s.set_option("autotune", 1)
+        if phases:
+            s.set_prephase(1.6, 1e-9, n_pre)
+        st = s.solve(w, n)
+        lam, hist = s.lambda_, s.residual_history(n)
+    R = O.divergence(d, w)
+    lam0 = O.sor(d, w, R, 1e-9, n_pre, omega=1.6)[0] if phases else None
+    L, it, _, ho = O.sor(d, w, R, 1e-9, n, lam=lam0, hist=True)
+    assert (st["iterations"], st["pre_iterations"]) == (it, n_pre * phases)
+    np.testing.assert_array_equal(lam, L)
+    np.testing.assert_array_equal(hist[:it], ho[:it])
+    for name, x in zip("uvw", O.correct(d, w, L)):
+        np.testing.assert_array_equal(getattr(w, name), x, err_msg=name)
+
+
 def test_autotune_restores_lambda_and_results_stay_exact(golden):
     d, w, z = golden("small_city.npz")
     lam0 = np.random.default_rng(7).standard_normal(d.numCellCentered()).astype(np.float32)
