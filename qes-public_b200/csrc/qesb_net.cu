@@ -136,29 +136,18 @@ struct ConvGeom {
   int Dc;       // depth of one item: D / Dc grids stacked along z, taps never cross from one to the next
 };
 
-// 16 bytes (8 channels c..c+7, never straddling x1/x2 since c1 % 16 == 0) of
-// the input at voxel (z, y, x) for an output voxel at depth zo, or zeros
-// outside the output voxel's item.
-__device__ __forceinline__ uint4 load_in8(const ConvIn &in, const ConvGeom &g, int zo, int z, int y, int x, int c)
-{
-  const int zb = zo - zo % g.Dc;
-  if (z < zb || z >= zb + g.Dc || y < 0 || y >= g.H || x < 0 || x >= g.W) return make_uint4(0, 0, 0, 0);
-  const __nv_bfloat16 *p;
-  if (c < in.c1) {
-    if (in.up1)
-      p = in.x1 + ((((long)(z >> 1) * (g.H >> 1) + (y >> 1)) * (g.W >> 1) + (x >> 1)) * in.c1 + c);
-    else
-      p = in.x1 + ((((long)z * g.H + y) * g.W + x) * in.c1 + c);
-  } else {
-    p = in.x2 + ((((long)z * g.H + y) * g.W + x) * in.c2 + (c - in.c1));
-  }
-  return __ldg(reinterpret_cast<const uint4 *>(p));
-}
-
 // 16-byte asynchronous copy global -> shared; valid = false fills zeros and reads nothing.
 __device__ __forceinline__ void cp16_zfill(void *dst, const void *src, bool valid)
 {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(umma::smem_u32(dst)), "l"(src),
+               "r"(valid ? 16 : 0)
+               : "memory");
+}
+
+// The same through L1, for gathers that read each voxel for several taps.
+__device__ __forceinline__ void cp16_zfill_l1(void *dst, const void *src, bool valid)
+{
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(umma::smem_u32(dst)), "l"(src),
                "r"(valid ? 16 : 0)
                : "memory");
 }
@@ -185,9 +174,12 @@ struct ConvOut {
 // the input at taps v + sign*offset(t), k = t*cin + c, Bm [N][Kp] K-major
 // BF16 (Kp = roundup(27*cin, 64), zero-padded). One CTA of 128 threads per
 // 128 voxels; a ring of NSTAGES shared-memory stages filled by asynchronous
-// 16-byte copies (zero-filled outside the grid) NSTAGES - 2 K chunks ahead,
+// 16-byte copies (zero-filled outside the grid) NSTAGES - 1 K chunks ahead,
 // so the gathers of the next chunks are in flight while chunk j's MMAs run;
-// accumulator N FP32 columns of TMEM.
+// accumulator N FP32 columns of TMEM. The gathers bound it: neighbouring taps
+// read the same voxels, so they go through L1 (past it, one 16 -> 16 channel
+// gradient on 64 x 64 x 32 voxels took 49 us, now 32; 32 -> 16: 66 and 46), and
+// one chunk ahead with 64-bit divisions per row it took 55 and 78.
 template <int N, int NSTAGES>
 __global__ void __launch_bounds__(128) k_conv_igemm(ConvIn in, ConvGeom g, int sign, const __nv_bfloat16 *__restrict__ Bm,
                                                    int Kp, ConvOut out, int *err)
@@ -196,7 +188,7 @@ __global__ void __launch_bounds__(128) k_conv_igemm(ConvIn in, ConvGeom g, int s
   // and stores its partial in slice y of out.acc; k_conv_finish adds the
   // slices in order and applies the epilogue (the same bits every run).
   constexpr uint32_t SA = 128 * 64 * 2, SB = N * 64 * 2, STAGE = SA + SB;
-  constexpr int NS = NSTAGES, DIST = NS - 2;  // chunk c's copies go out DIST iterations before its MMAs
+  constexpr int NS = NSTAGES, DIST = NS - 1;  // chunk c's copies go out DIST iterations before its MMAs
   constexpr uint32_t NCOLS = N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : 256;
   extern __shared__ __align__(1024) uint8_t sm[];
   __shared__ __align__(8) uint64_t mbar[NS];  // stage s: the MMAs of chunk c, c % NS == s
@@ -217,64 +209,77 @@ __global__ void __launch_bounds__(128) k_conv_igemm(ConvIn in, ConvGeom g, int s
   const uint32_t tmem = tmem_base;
   constexpr uint32_t idesc = umma::idesc_bf16(128, N, 0, 0);
 
-  // this thread's 8 rows (m = tid/8 + 16 i) and fixed k-group g = tid % 8
-  const int g8 = tid & 7;
-  int rz[8], ry[8], rx[8], rzb[8];
-  long rvox[8];
-  bool rv[8];
+  // this thread's 8 rows m = r0 + 16 i and its k-group g8: eight consecutive rows are eight lanes, whose 16-byte
+  // copies fill 128 bytes of shared memory in a row (k-groups lie 128 bytes apart: eight of them conflict eightfold)
+  const int g8 = tid >> 3 & 7, r0 = (tid & 7) | tid >> 6 << 3;
+  // (16 voxels apart: one division, then additions), and which taps of each stay in its item: bit 1 + d of
+  // three bits each for z, y and x
+  int rz[8], ry[8], rx[8], rin[8];
+  const long vox0 = m0 + r0;
+  {
+    int x = (int)(vox0 % g.W), y = (int)((vox0 / g.W) % g.H), z = (int)(vox0 / ((long)g.W * g.H)), dc = z % g.Dc;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const long v = m0 + (tid >> 3) + 16 * i;
-    rv[i] = v < g.V;
-    const long vv = rv[i] ? v : 0;
-    rvox[i] = vv;
-    rx[i] = (int)(vv % g.W);
-    ry[i] = (int)((vv / g.W) % g.H);
-    rz[i] = (int)(vv / ((long)g.W * g.H));
-    rzb[i] = rz[i] - rz[i] % g.Dc;  // the row's item starts at this depth
+    for (int i = 0; i < 8; ++i) {
+      rz[i] = z;
+      ry[i] = y;
+      rx[i] = x;
+      rin[i] = vox0 + 16 * i < g.V ? (dc > 0) | 2 | (dc + 1 < g.Dc) << 2 | (y > 0) << 3 | 16 | (y + 1 < g.H) << 5 |
+                                         (x > 0) << 6 | 128 | (x + 1 < g.W) << 8
+                                   : 0;
+      x += 16;
+      while (x >= g.W) {
+        x -= g.W;
+        if (++y == g.H) {
+          y = 0;
+          ++z;
+          if (++dc == g.Dc) dc = 0;
+        }
+      }
+    }
   }
   const int nk_all = Kp / 64, per = (nk_all + gridDim.y - 1) / gridDim.y;
   const int jb = blockIdx.y * per, je = min(nk_all, jb + per), nk = je > jb ? je - jb : 0;
-  // this thread's copies of local chunk jl into its stage (one commit group, empty past the range)
+  int kt = (jb * 64 + 8 * g8) / cin, kc = jb * 64 + 8 * g8 - kt * cin;  // tap and channel of this thread's next copies
+  // this thread's copies of local chunk jl (in turn) into its stage (one commit group, empty past the range)
   auto issue = [&](int jl) {
     if (jl < nk) {
       const int j = jb + jl;
       uint8_t *sa = sm + (jl % NS) * STAGE, *sb = sa + SA;
-      // A: rows m = tid/8 + 16 i, k-group g8
-      const int kk = j * 64 + 8 * g8;
-      const int t = kk / cin, c = kk - t * cin;
+      const int t = kt, c = kc;
+      for (kc += 64; kc >= cin; kc -= cin) ++kt;
       int dz = 0, dy = 0, dx = 0;
       if (t < 27) tap_offset(t, dz, dy, dx);
       dz *= sign;
       dy *= sign;
       dx *= sign;
+      auto inside = [&](int i) {
+        return t < 27 && (rin[i] >> (dz + 1) & rin[i] >> (dy + 4) & rin[i] >> (dx + 7) & 1) != 0;
+      };
       if (in.up1 && c < in.c1) {  // the upsampled input: the coarse voxel of each fine one
         const int Hc = g.H >> 1, Wc = g.W >> 1;
         const __nv_bfloat16 *tb = in.x1 + c;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int z = rz[i] + dz, y = ry[i] + dy, x = rx[i] + dx;
-          const bool valid = rv[i] && t < 27 && z >= rzb[i] && z < rzb[i] + g.Dc && (unsigned)y < (unsigned)g.H &&
-                             (unsigned)x < (unsigned)g.W;
+          const bool valid = inside(i);
           const long cv = ((long)(z >> 1) * Hc + (y >> 1)) * Wc + (x >> 1);
-          cp16_zfill(sa + off_kmajor((tid >> 3) + 16 * i, 8 * g8), valid ? tb + cv * in.c1 : in.x1, valid);
+          cp16_zfill_l1(sa + off_kmajor(r0 + 16 * i, 8 * g8), valid ? tb + cv * in.c1 : in.x1, valid);
         }
       } else {  // same-grid input: one voxel offset for the tap, bounds per row
         const long dv = ((long)dz * g.H + dy) * g.W + dx;
         const bool first = c < in.c1;
-        const __nv_bfloat16 *tb = first ? in.x1 + c : in.x2 + (c - in.c1);
+        const __nv_bfloat16 *tb = first ? in.x1 + c : in.x2 + (c - in.c1);  // this thread's first row, then every 16th
         const int cs = first ? in.c1 : in.c2;
+        tb += (vox0 + dv) * cs;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const int z = rz[i] + dz, y = ry[i] + dy, x = rx[i] + dx;
-          const bool valid = rv[i] && t < 27 && z >= rzb[i] && z < rzb[i] + g.Dc && (unsigned)y < (unsigned)g.H &&
-                             (unsigned)x < (unsigned)g.W;
-          cp16_zfill(sa + off_kmajor((tid >> 3) + 16 * i, 8 * g8), valid ? tb + (rvox[i] + dv) * cs : in.x1, valid);
+          const bool valid = inside(i);
+          cp16_zfill_l1(sa + off_kmajor(r0 + 16 * i, 8 * g8), valid ? tb + 16 * i * cs : in.x1, valid);
         }
       }
       // B: N rows x 8 k-groups
       for (int idx = tid; idx < N * 8; idx += 128) {
-        const int n = idx >> 3, gg = idx & 7;
+        const int n = (idx & 7) | idx >> 6 << 3, gg = idx >> 3 & 7;
         cp16_zfill(sb + off_kmajor(n, 8 * gg), Bm + (long)n * Kp + j * 64 + 8 * gg, true);
       }
     }
@@ -282,15 +287,13 @@ __global__ void __launch_bounds__(128) k_conv_igemm(ConvIn in, ConvGeom g, int s
   };
   bool ok = true;
   for (int jl = 0; jl < DIST; ++jl) issue(jl);
-  for (int jl = 0; jl < nk && ok; ++jl) {
-    // refill the stage chunk jl + DIST - NS used (its MMAs were issued two iterations ago)
-    const int c = jl + DIST - NS;
-    if (c >= 0) ok = umma::mbar_wait(&mbar[c % NS], (c / NS) & 1, kWaitLimit);
-    if (!ok) break;
-    issue(jl + DIST);
-    asm volatile("cp.async.wait_group %0;" ::"n"(DIST) : "memory");  // chunk jl's copies (this thread's) landed
+  for (int jl = 0; jl < nk; ++jl) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(DIST - 1) : "memory");  // chunk jl's copies (this thread's) landed
     umma::fence_smem_async();
-    __syncthreads();  // everyone's
+    if (__syncthreads_or(!ok)) {  // everyone's; and no one's wait gave up
+      ok = false;
+      break;
+    }
     if (tid == 0) {
       umma::fence_after_sync();
       const uint32_t a0 = umma::smem_u32(sm + (jl % NS) * STAGE), b0 = a0 + SA;
@@ -300,6 +303,9 @@ __global__ void __launch_bounds__(128) k_conv_igemm(ConvIn in, ConvGeom g, int s
                        (jl > 0 || kk > 0) ? 1u : 0u);
       umma::mma_commit(&mbar[jl % NS]);
     }
+    // refill the stage that the MMAs of chunk jl - 1 have read
+    if (jl >= 1 && jl + DIST < nk) ok = umma::mbar_wait(&mbar[(jl - 1) % NS], ((jl - 1) / NS) & 1, kWaitLimit);
+    if (ok) issue(jl + DIST);
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");  // no copy outlives the CTA's shared memory
   if (ok && nk > 0) ok = umma::mbar_wait(&mbar[(nk - 1) % NS], ((nk - 1) / NS) & 1, kWaitLimit);
@@ -1159,8 +1165,8 @@ __global__ void __launch_bounds__(192, 1) k_conv_zflat3(const __grid_constant__ 
 // meet in dW (FP32) by atomic adds, four floats each where dW is aligned.
 // The gather bounds it (27 taps of 16 bytes a voxel and 8 channels): loads that
 // each chunk waits for, divisions for every voxel and scalar atomics took
-// 103 us for 16 -> 16 channels on 64 x 64 x 32 voxels, this form takes 53;
-// 64 + 32 -> 32 channels on 32 x 32 x 16: 161 and 45.
+// 103 us for 16 -> 16 channels on 64 x 64 x 32 voxels, this form takes 43 (54
+// with the copies past L1); 64 + 32 -> 32 channels on 32 x 32 x 16: 161 and 37.
 constexpr int kWgStages = 3;
 template <int N>
 __global__ void __launch_bounds__(128) k_conv_wgrad(ConvIn in, ConvGeom g, const __nv_bfloat16 *__restrict__ dY,
@@ -1220,7 +1226,7 @@ __global__ void __launch_bounds__(128) k_conv_wgrad(ConvIn in, ConvGeom g, const
         else if (in.up1) p = in.x1 + (((long)(zz >> 1) * (g.H >> 1) + (yy >> 1)) * (g.W >> 1) + (xx >> 1)) * in.c1 + c;
         else p = in.x1 + (((long)zz * g.H + yy) * g.W + xx) * in.c1 + c;
       }
-      cp16_zfill(sa + off_mnmajor(8 * ((tid >> 6) + 2 * i), kv, 128), p, in_);
+      cp16_zfill_l1(sa + off_mnmajor(8 * ((tid >> 6) + 2 * i), kv, 128), p, in_);
     }
     for (int idx = tid; idx < N / 8 * 64; idx += 128) {
       const int ng = idx >> 6, k = idx & 63;
@@ -1410,7 +1416,7 @@ template <int N>
 qesb_status launch_conv(const ConvIn &in, const ConvGeom &g, int sign, const __nv_bfloat16 *Bm, int Kp,
                         const ConvOut &out, int *err, cudaStream_t s)
 {
-  // three stages (gathers one chunk ahead, three CTAs per SM at N = 32), or four (two ahead) on conv path 5
+  // three stages (gathers two chunks ahead, three CTAs per SM at N = 32), or four (three ahead) on conv path 5
   const bool three = g_conv_path != 5;
   const int smem = (three ? 3 : 4) * (128 * 64 * 2 + N * 64 * 2);
   int dev = 0;

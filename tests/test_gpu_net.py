@@ -171,6 +171,26 @@ def test_conv3d_weight_gradient(D, H, W, ci, co, up):
     np.testing.assert_allclose(dW.view(27 * cin, co).cpu().double().numpy(), ref.numpy(), rtol=1e-4, atol=1e-3)
 
 
+# The implicit GEMM's walk over its rows: rows of 1 to 130 voxels, ragged last
+# tiles, a tap's channels within one 64-wide chunk and across several, split and
+# unsplit sums, both tap directions. Exact products of order 1 / sqrt(K) summed
+# in FP32: 1e-4.
+@pytest.mark.parametrize("sign", [1, -1])
+@pytest.mark.parametrize("D,H,W,ci,co", [(5, 7, 1, 16, 16), (3, 4, 3, 48, 32), (9, 2, 17, 32, 16), (2, 3, 130, 80, 64),
+                                         (31, 37, 33, 16, 16), (1, 1, 1, 128, 128)])
+def test_conv3d_gemm_row_walk(conv_path, D, H, W, ci, co, sign):
+    import torch
+    torch.manual_seed(W + ci)
+    x = _bf16(torch.randn(1, ci, D, H, W))
+    w = _bf16(torch.randn(co, ci, 3, 3, 3) / (27 * ci) ** 0.5)
+    wt = w.double() if sign == 1 else w.double().flip(2, 3, 4)
+    ref = _cl(torch.nn.functional.conv3d(x.double(), wt, padding=1)).numpy()
+    bm, kp = _bm_forward(w)
+    conv_path(1)
+    out = _run_conv(_cl(x).to("cuda:0"), ci, 0, None, 0, D, H, W, sign, bm.to("cuda:0"), kp, co).numpy()
+    np.testing.assert_allclose(out, ref, rtol=1e-4, atol=1e-4)
+
+
 # Rows shorter and longer than a 64-voxel chunk, ragged last chunks, one to nine
 # chunks a CTA, dW on and off a 16-byte boundary. The BF16 products are exact in
 # FP32, so the error is that of summing V of them in any order: below
