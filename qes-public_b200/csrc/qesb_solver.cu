@@ -3086,73 +3086,73 @@ qesb_status qesb_solve_batch(qesb_handle *const *hs, int n, int itermax, float *
   qesb_status qs = QESB_OK;
   int launched = 0, pre_launched = 0;
   if (ns > 0) {
-  k_sweep_stamp<<<1, 1, 0, s>>>(list.a.ctl);  // the latencies (ms_sor) count from here
-  CK(cudaEventRecord(h0->evs[0], s));
-  if (!start.empty()) {
-    // the start stages of the pre-phases that have one, as a list of their own
-    sweep_tiles(start, sv, true, h0->device);
-    qs = list.upload(start, sv.unit, s);
-    int smax = 0;
-    for (int i : start_of) smax = std::max(smax, hs[i]->start_iters);
-    int n1 = 0;
-    if (qs == QESB_OK)
-      qs = run_sweep_loop(sv, true, list.a, h0->device, s, cells, smax, h0->opt_graph != 0, &h0->bgraph_start,
-                          h0->h_ctl, h0->h_ctl_dev, &n1, 0, 1, h0->opt_pdl != 0);
-    pre_launched += n1;
-    for (size_t q = 0; q < start_of.size() && qs == QESB_OK; ++q)
-      qs = wb.add(hs[start_of[q]]->h_state_dev, hs[start_of[q]]->d_state, sizeof(SolveState));
-    if (qs == QESB_OK) qs = wb.flush();
-    if (qs == QESB_OK) CK(cudaStreamSynchronize(s));
-    for (size_t q = 0; q < start_of.size() && qs == QESB_OK; ++q) {
-      qesb_handle *h = hs[start_of[q]];
-      const SolveState sp = *h->h_state;
-      if (sp.nan)
-        qs = qesb_fail(QESB_ERR_NUMERIC, "NaN in lambda of batch domain %d during the pre-phase's start stage",
-                       start_of[q]);
-      h->last_pre_iterations = sp.it;
-      if (qs == QESB_OK) qs = wb.zero(h->d_err, sizeof(double) * err_slots(h, itermax));
-      if (qs == QESB_OK) qs = wb.zero(h->d_state, sizeof(SolveState));
+    k_sweep_stamp<<<1, 1, 0, s>>>(list.a.ctl);  // the latencies (ms_sor) count from here
+    CK(cudaEventRecord(h0->evs[0], s));
+    if (!start.empty()) {
+      // the start stages of the pre-phases that have one, as a list of their own
+      sweep_tiles(start, sv, true, h0->device);
+      qs = list.upload(start, sv.unit, s);
+      int smax = 0;
+      for (int i : start_of) smax = std::max(smax, hs[i]->start_iters);
+      int n1 = 0;
+      if (qs == QESB_OK)
+        qs = run_sweep_loop(sv, true, list.a, h0->device, s, cells, smax, h0->opt_graph != 0, &h0->bgraph_start,
+                            h0->h_ctl, h0->h_ctl_dev, &n1, 0, 1, h0->opt_pdl != 0);
+      pre_launched += n1;
+      for (size_t q = 0; q < start_of.size() && qs == QESB_OK; ++q)
+        qs = wb.add(hs[start_of[q]]->h_state_dev, hs[start_of[q]]->d_state, sizeof(SolveState));
+      if (qs == QESB_OK) qs = wb.flush();
+      if (qs == QESB_OK) CK(cudaStreamSynchronize(s));
+      for (size_t q = 0; q < start_of.size() && qs == QESB_OK; ++q) {
+        qesb_handle *h = hs[start_of[q]];
+        const SolveState sp = *h->h_state;
+        if (sp.nan)
+          qs = qesb_fail(QESB_ERR_NUMERIC, "NaN in lambda of batch domain %d during the pre-phase's start stage",
+                         start_of[q]);
+        h->last_pre_iterations = sp.it;
+        if (qs == QESB_OK) qs = wb.zero(h->d_err, sizeof(double) * err_slots(h, itermax));
+        if (qs == QESB_OK) qs = wb.zero(h->d_state, sizeof(SolveState));
+      }
+      if (qs == QESB_OK) qs = wb.flush();
     }
-    if (qs == QESB_OK) qs = wb.flush();
-  }
-  if (!pre.empty() && qs == QESB_OK) {
-    // the over-relaxed pre-phase of the domains that have one, as a list of its own
-    sweep_tiles(pre, sv, true, h0->device);
-    qs = list.upload(pre, sv.unit, s);
-    int pre_max = 0;
-    for (int i : pre_of) pre_max = std::max(pre_max, hs[i]->pre_iters);
-    int n2 = 0;
-    if (qs == QESB_OK)
-      qs = run_sweep_loop(sv, true, list.a, h0->device, s, cells, pre_max, h0->opt_graph != 0, &h0->bgraph_pre,
-                          h0->h_ctl, h0->h_ctl_dev, &n2, 0, 1, h0->opt_pdl != 0);
-    pre_launched += n2;
-    for (size_t q = 0; q < pre_of.size() && qs == QESB_OK; ++q)
-      qs = wb.add(hs[pre_of[q]]->h_state_dev, hs[pre_of[q]]->d_state, sizeof(SolveState));
-    if (qs == QESB_OK) qs = wb.flush();
-    if (qs == QESB_OK) CK(cudaStreamSynchronize(s));
-    for (size_t q = 0; q < pre_of.size() && qs == QESB_OK; ++q) {
-      qesb_handle *h = hs[pre_of[q]];
-      const SolveState sp = *h->h_state;
-      if (sp.nan) qs = qesb_fail(QESB_ERR_NUMERIC, "NaN in lambda of batch domain %d during the pre-phase", pre_of[q]);
-      h->last_pre_iterations += sp.it;
-      if (qs == QESB_OK) qs = wb.zero(h->d_err, sizeof(double) * std::max(itermax, 1));
-      if (qs == QESB_OK) qs = wb.zero(h->d_state, sizeof(SolveState));
+    if (!pre.empty() && qs == QESB_OK) {
+      // the over-relaxed pre-phase of the domains that have one, as a list of its own
+      sweep_tiles(pre, sv, true, h0->device);
+      qs = list.upload(pre, sv.unit, s);
+      int pre_max = 0;
+      for (int i : pre_of) pre_max = std::max(pre_max, hs[i]->pre_iters);
+      int n2 = 0;
+      if (qs == QESB_OK)
+        qs = run_sweep_loop(sv, true, list.a, h0->device, s, cells, pre_max, h0->opt_graph != 0, &h0->bgraph_pre,
+                            h0->h_ctl, h0->h_ctl_dev, &n2, 0, 1, h0->opt_pdl != 0);
+      pre_launched += n2;
+      for (size_t q = 0; q < pre_of.size() && qs == QESB_OK; ++q)
+        qs = wb.add(hs[pre_of[q]]->h_state_dev, hs[pre_of[q]]->d_state, sizeof(SolveState));
+      if (qs == QESB_OK) qs = wb.flush();
+      if (qs == QESB_OK) CK(cudaStreamSynchronize(s));
+      for (size_t q = 0; q < pre_of.size() && qs == QESB_OK; ++q) {
+        qesb_handle *h = hs[pre_of[q]];
+        const SolveState sp = *h->h_state;
+        if (sp.nan) qs = qesb_fail(QESB_ERR_NUMERIC, "NaN in lambda of batch domain %d during the pre-phase", pre_of[q]);
+        h->last_pre_iterations += sp.it;
+        if (qs == QESB_OK) qs = wb.zero(h->d_err, sizeof(double) * std::max(itermax, 1));
+        if (qs == QESB_OK) qs = wb.zero(h->d_state, sizeof(SolveState));
+      }
+      if (qs == QESB_OK) qs = wb.flush();
     }
-    if (qs == QESB_OK) qs = wb.flush();
-  }
-  CK(cudaEventRecord(h0->evs[1], s));
-  sweep_tiles(doms, sv, true, h0->device);
-  if (qs == QESB_OK) qs = list.upload(doms, sv.unit, s);
-  if (qs == QESB_OK && h0->win_k > 0)  // each domain's first window starts from lambda as the loop begins
-    for (size_t q = 0; q < str_of.size() && qs == QESB_OK; ++q)
-      qs = copy_floats(hs[str_of[q]]->d_snap, hs[str_of[q]]->d_lam_s, 2L * hs[str_of[q]]->S.CS, s);
-  if (qs == QESB_OK) {
-    CK(cudaEventRecord(h0->evs[2], s));
-    if (itermax > 0)
-      qs = run_sweep_loop(sv, true, list.a, h0->device, s, cells, itermax, h0->opt_graph != 0, &h0->bgraph, h0->h_ctl,
-                          h0->h_ctl_dev, &launched, h0->win_k, ns, h0->opt_pdl != 0);
-    CK(cudaEventRecord(h0->evs[3], s));
-  }
+    CK(cudaEventRecord(h0->evs[1], s));
+    sweep_tiles(doms, sv, true, h0->device);
+    if (qs == QESB_OK) qs = list.upload(doms, sv.unit, s);
+    if (qs == QESB_OK && h0->win_k > 0)  // each domain's first window starts from lambda as the loop begins
+      for (size_t q = 0; q < str_of.size() && qs == QESB_OK; ++q)
+        qs = copy_floats(hs[str_of[q]]->d_snap, hs[str_of[q]]->d_lam_s, 2L * hs[str_of[q]]->S.CS, s);
+    if (qs == QESB_OK) {
+      CK(cudaEventRecord(h0->evs[2], s));
+      if (itermax > 0)
+        qs = run_sweep_loop(sv, true, list.a, h0->device, s, cells, itermax, h0->opt_graph != 0, &h0->bgraph, h0->h_ctl,
+                            h0->h_ctl_dev, &launched, h0->win_k, ns, h0->opt_pdl != 0);
+      CK(cudaEventRecord(h0->evs[3], s));
+    }
   }
   const unsigned long long t0 = ns > 0 ? h0->h_ctl->t0 : 0;
   CK(cudaEventRecord(h0->ev[2], s));
