@@ -172,16 +172,17 @@ struct ConvOut {
 
 // Y[v][n] = epilogue( sum_k A[v][k] * Bm[n][k] ), A the implicit im2col of
 // the input at taps v + sign*offset(t), k = t*cin + c, Bm [N][Kp] K-major
-// BF16 (Kp = roundup(27*cin, 64), zero-padded). One CTA of 128 threads per
+// BF16 (Kp = roundup(27*cin, 64), zero-padded). One CTA of 256 threads per
 // 128 voxels; a ring of NSTAGES shared-memory stages filled by asynchronous
 // 16-byte copies (zero-filled outside the grid) NSTAGES - 1 K chunks ahead,
 // so the gathers of the next chunks are in flight while chunk j's MMAs run;
 // accumulator N FP32 columns of TMEM. The gathers bound it: neighbouring taps
 // read the same voxels, so they go through L1 (past it, one 16 -> 16 channel
-// gradient on 64 x 64 x 32 voxels took 49 us, now 32; 32 -> 16: 66 and 46), and
-// one chunk ahead with 64-bit divisions per row it took 55 and 78.
+// gradient on 64 x 64 x 32 voxels took 49 us, now 31; 16 -> 32: 66 and 43), and
+// one chunk ahead with 64-bit divisions per row it took 55 and 78. 128 threads
+// a CTA (twice the address arithmetic in each, between the copies): 32 and 46.
 template <int N, int NSTAGES>
-__global__ void __launch_bounds__(128) k_conv_igemm(ConvIn in, ConvGeom g, int sign, const __nv_bfloat16 *__restrict__ Bm,
+__global__ void __launch_bounds__(256) k_conv_igemm(ConvIn in, ConvGeom g, int sign, const __nv_bfloat16 *__restrict__ Bm,
                                                    int Kp, ConvOut out, int *err)
 {
   // split-K (gridDim.y > 1, small grids): CTA y sums the K chunks [jb, je)
@@ -209,24 +210,24 @@ __global__ void __launch_bounds__(128) k_conv_igemm(ConvIn in, ConvGeom g, int s
   const uint32_t tmem = tmem_base;
   constexpr uint32_t idesc = umma::idesc_bf16(128, N, 0, 0);
 
-  // this thread's 8 rows m = r0 + 16 i and its k-group g8: eight consecutive rows are eight lanes, whose 16-byte
+  // this thread's 4 rows m = r0 + 32 i and its k-group g8: eight consecutive rows are eight lanes, whose 16-byte
   // copies fill 128 bytes of shared memory in a row (k-groups lie 128 bytes apart: eight of them conflict eightfold)
   const int g8 = tid >> 3 & 7, r0 = (tid & 7) | tid >> 6 << 3;
-  // (16 voxels apart: one division, then additions), and which taps of each stay in its item: bit 1 + d of
+  // (32 voxels apart: one division, then additions), and which taps of each stay in its item: bit 1 + d of
   // three bits each for z, y and x
-  int rz[8], ry[8], rx[8], rin[8];
+  int rz[4], ry[4], rx[4], rin[4];
   const long vox0 = m0 + r0;
   {
     int x = (int)(vox0 % g.W), y = (int)((vox0 / g.W) % g.H), z = (int)(vox0 / ((long)g.W * g.H)), dc = z % g.Dc;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < 4; ++i) {
       rz[i] = z;
       ry[i] = y;
       rx[i] = x;
-      rin[i] = vox0 + 16 * i < g.V ? (dc > 0) | 2 | (dc + 1 < g.Dc) << 2 | (y > 0) << 3 | 16 | (y + 1 < g.H) << 5 |
+      rin[i] = vox0 + 32 * i < g.V ? (dc > 0) | 2 | (dc + 1 < g.Dc) << 2 | (y > 0) << 3 | 16 | (y + 1 < g.H) << 5 |
                                          (x > 0) << 6 | 128 | (x + 1 < g.W) << 8
                                    : 0;
-      x += 16;
+      x += 32;
       while (x >= g.W) {
         x -= g.W;
         if (++y == g.H) {
@@ -259,26 +260,26 @@ __global__ void __launch_bounds__(128) k_conv_igemm(ConvIn in, ConvGeom g, int s
         const int Hc = g.H >> 1, Wc = g.W >> 1;
         const __nv_bfloat16 *tb = in.x1 + c;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < 4; ++i) {
           const int z = rz[i] + dz, y = ry[i] + dy, x = rx[i] + dx;
           const bool valid = inside(i);
           const long cv = ((long)(z >> 1) * Hc + (y >> 1)) * Wc + (x >> 1);
-          cp16_zfill_l1(sa + off_kmajor(r0 + 16 * i, 8 * g8), valid ? tb + cv * in.c1 : in.x1, valid);
+          cp16_zfill_l1(sa + off_kmajor(r0 + 32 * i, 8 * g8), valid ? tb + cv * in.c1 : in.x1, valid);
         }
       } else {  // same-grid input: one voxel offset for the tap, bounds per row
         const long dv = ((long)dz * g.H + dy) * g.W + dx;
         const bool first = c < in.c1;
-        const __nv_bfloat16 *tb = first ? in.x1 + c : in.x2 + (c - in.c1);  // this thread's first row, then every 16th
+        const __nv_bfloat16 *tb = first ? in.x1 + c : in.x2 + (c - in.c1);  // this thread's first row, then every 32nd
         const int cs = first ? in.c1 : in.c2;
         tb += (vox0 + dv) * cs;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < 4; ++i) {
           const bool valid = inside(i);
-          cp16_zfill_l1(sa + off_kmajor(r0 + 16 * i, 8 * g8), valid ? tb + 16 * i * cs : in.x1, valid);
+          cp16_zfill_l1(sa + off_kmajor(r0 + 32 * i, 8 * g8), valid ? tb + 32 * i * cs : in.x1, valid);
         }
       }
       // B: N rows x 8 k-groups
-      for (int idx = tid; idx < N * 8; idx += 128) {
+      for (int idx = tid; idx < N * 8; idx += 256) {
         const int n = (idx & 7) | idx >> 6 << 3, gg = idx >> 3 & 7;
         cp16_zfill(sb + off_kmajor(n, 8 * gg), Bm + (long)n * Kp + j * 64 + 8 * gg, true);
       }
@@ -314,20 +315,20 @@ __global__ void __launch_bounds__(128) k_conv_igemm(ConvIn in, ConvGeom g, int s
     if (lane == 0) atomicExch(err, 1);
     umma::mma_drain(&mdrain, tid == 0, kWaitLimit);
   } else if (out.acc) {
-    const long v = m0 + warp * 32 + lane;
-    for (int c0 = 0; c0 < N; c0 += 8) {
+    const long v = m0 + (warp & 3) * 32 + lane;
+    for (int c0 = (warp >> 2) * (N / 2); c0 < ((warp >> 2) + 1) * (N / 2); c0 += 8) {
       float a[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // an empty K range contributes zeros
-      if (nk > 0) umma::tmem_ld8(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, a);
+      if (nk > 0) umma::tmem_ld8(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, a);
       if (v < g.V) {
 #pragma unroll
         for (int q = 0; q < 8; ++q) out.acc[((long)blockIdx.y * g.V + v) * N + c0 + q] = a[q];
       }
     }
   } else {
-    const long v = m0 + warp * 32 + lane;
-    for (int c0 = 0; c0 < N; c0 += 8) {
+    const long v = m0 + (warp & 3) * 32 + lane;
+    for (int c0 = (warp >> 2) * (N / 2); c0 < ((warp >> 2) + 1) * (N / 2); c0 += 8) {
       float a[8];
-      umma::tmem_ld8(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, a);
+      umma::tmem_ld8(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, a);
       if (v < g.V) {
         if (out.bias) {
 #pragma unroll
@@ -1165,11 +1166,12 @@ __global__ void __launch_bounds__(192, 1) k_conv_zflat3(const __grid_constant__ 
 // meet in dW (FP32) by atomic adds, four floats each where dW is aligned.
 // The gather bounds it (27 taps of 16 bytes a voxel and 8 channels): loads that
 // each chunk waits for, divisions for every voxel and scalar atomics took
-// 103 us for 16 -> 16 channels on 64 x 64 x 32 voxels, this form takes 43 (54
-// with the copies past L1); 64 + 32 -> 32 channels on 32 x 32 x 16: 161 and 37.
+// 103 us for 16 -> 16 channels on 64 x 64 x 32 voxels, this form takes 42 (54
+// with the copies past L1, 43 with 128 threads); 64 + 32 -> 32 channels on
+// 32 x 32 x 16: 161 and 36.
 constexpr int kWgStages = 3;
 template <int N>
-__global__ void __launch_bounds__(128) k_conv_wgrad(ConvIn in, ConvGeom g, const __nv_bfloat16 *__restrict__ dY,
+__global__ void __launch_bounds__(256) k_conv_wgrad(ConvIn in, ConvGeom g, const __nv_bfloat16 *__restrict__ dY,
                                                    long vchunk, float *__restrict__ dW, int *err)
 {
   constexpr uint32_t SA = 128 * 64 * 2, SB = N * 64 * 2, STAGE = SA + SB;
@@ -1196,13 +1198,13 @@ __global__ void __launch_bounds__(128) k_conv_wgrad(ConvIn in, ConvGeom g, const
   umma::fence_after_sync();
   const uint32_t tmem = tmem_base;
   constexpr uint32_t idesc = umma::idesc_bf16(128, N, 1, 1);
-  // this thread: voxel column kv = tid % 64 of each chunk; row groups rg = tid/64 + 2 i: their tap (packed, 2 bits
+  // this thread: voxel column kv = tid % 64 of each chunk; row groups rg = tid/64 + 4 i: their tap (packed, 2 bits
   // an axis; -1: none) and channel
   const int kv = tid & 63;
-  int tg[8], cg[8];
+  int tg[4], cg[4];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int m = mt0 + 8 * ((tid >> 6) + 2 * i);
+  for (int i = 0; i < 4; ++i) {
+    const int m = mt0 + 8 * ((tid >> 6) + 4 * i);
     const int t = m / cin;
     tg[i] = m < Mrows ? (t / 9) << 4 | (t / 3 % 3) << 2 | t % 3 : -1;
     cg[i] = m < Mrows ? m - t * cin : 0;
@@ -1216,7 +1218,7 @@ __global__ void __launch_bounds__(128) k_conv_wgrad(ConvIn in, ConvGeom g, const
     uint8_t *sa = sm + (j % kWgStages) * STAGE, *sb = sa + SA;
     const bool vin = v < ve;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < 4; ++i) {
       const int zz = z + (tg[i] >> 4) - 1, yy = y + (tg[i] >> 2 & 3) - 1, xx = x + (tg[i] & 3) - 1, c = cg[i];
       const bool in_ = vin && tg[i] >= 0 && zz >= zb && zz < zb + g.Dc && (unsigned)yy < (unsigned)g.H &&
                        (unsigned)xx < (unsigned)g.W;
@@ -1226,9 +1228,9 @@ __global__ void __launch_bounds__(128) k_conv_wgrad(ConvIn in, ConvGeom g, const
         else if (in.up1) p = in.x1 + (((long)(zz >> 1) * (g.H >> 1) + (yy >> 1)) * (g.W >> 1) + (xx >> 1)) * in.c1 + c;
         else p = in.x1 + (((long)zz * g.H + yy) * g.W + xx) * in.c1 + c;
       }
-      cp16_zfill_l1(sa + off_mnmajor(8 * ((tid >> 6) + 2 * i), kv, 128), p, in_);
+      cp16_zfill_l1(sa + off_mnmajor(8 * ((tid >> 6) + 4 * i), kv, 128), p, in_);
     }
-    for (int idx = tid; idx < N / 8 * 64; idx += 128) {
+    for (int idx = tid; idx < N / 8 * 64; idx += 256) {
       const int ng = idx >> 6, k = idx & 63;
       const long vv = vb + (long)j * 64 + k;
       cp16_zfill(sb + off_mnmajor(8 * ng, k, N), vv < ve ? dY + vv * N + 8 * ng : dY, vv < ve);
@@ -1281,11 +1283,11 @@ __global__ void __launch_bounds__(128) k_conv_wgrad(ConvIn in, ConvGeom g, const
     if (lane == 0) atomicExch(err, 1);
     umma::mma_drain(&mdrain, tid == 0, kWaitLimit);
   } else {
-    const int m = mt0 + warp * 32 + lane;
+    const int m = mt0 + (warp & 3) * 32 + lane;
     const bool al16 = (reinterpret_cast<uintptr_t>(dW) & 15) == 0;
-    for (int c0 = 0; c0 < N; c0 += 8) {
+    for (int c0 = (warp >> 2) * (N / 2); c0 < ((warp >> 2) + 1) * (N / 2); c0 += 8) {
       float a[8];
-      umma::tmem_ld8(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, a);
+      umma::tmem_ld8(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, a);
       if (m < Mrows && !al16) {
 #pragma unroll
         for (int q = 0; q < 8; ++q) atomicAdd(dW + (long)m * N + c0 + q, a[q]);
@@ -1440,8 +1442,8 @@ qesb_status launch_conv(const ConvIn &in, const ConvGeom &g, int sign, const __n
     const qesb_status st = acc_buffer(dev, s, need, &o.acc);
     if (st != QESB_OK) return st;
   }
-  if (three) k_conv_igemm<N, 3><<<dim3(blocks, split), 128, smem, s>>>(in, g, sign, Bm, Kp, o, err);
-  else k_conv_igemm<N, 4><<<dim3(blocks, split), 128, smem, s>>>(in, g, sign, Bm, Kp, o, err);
+  if (three) k_conv_igemm<N, 3><<<dim3(blocks, split), 256, smem, s>>>(in, g, sign, Bm, Kp, o, err);
+  else k_conv_igemm<N, 4><<<dim3(blocks, split), 256, smem, s>>>(in, g, sign, Bm, Kp, o, err);
   if (split > 1) {
     launch_finish(o.acc, split, g.V, N, out, s);
   }
@@ -1683,7 +1685,7 @@ qesb_status launch_wgrad(const ConvIn &in, const ConvGeom &g, const __nv_bfloat1
   }
   const int cin = in.c1 + in.c2;
   const dim3 grid((unsigned)((27 * cin + 127) / 128), (unsigned)((g.V + vchunk - 1) / vchunk));
-  k_conv_wgrad<N><<<grid, 128, smem, s>>>(in, g, dY, vchunk, dW, err);
+  k_conv_wgrad<N><<<grid, 256, smem, s>>>(in, g, dY, vchunk, dW, err);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? QESB_OK : qesb_fail(QESB_ERR_CUDA, "wgrad launch: %s", cudaGetErrorString(e));
 }

@@ -177,7 +177,7 @@ class WarmStartNet:
         D, H, W = s.level(lvl)
         V = D * H * W
         # about three CTAs an SM over the kernel's 128-row tiles: fewer leave SMs idle, more only add partial sums
-        # (16 -> 16 channels on 64 x 64 x 32: 43 us at 1024 voxels a CTA, 50 at 256, 66 at 2048)
+        # (16 -> 16 channels on 64 x 64 x 32: 42 us at 1024 voxels a CTA, 50 at 2048, 93 at 64)
         tiles = (27 * (L.c1 + L.c2) + 127) // 128
         vchunk = max(64, min(8192, (tiles * V // (3 * 148) + 63) // 64 * 64))
         check(lib().qesb_conv3d_wgrad(_p(x1), L.c1, L.up1, _p(x2), L.c2, D, H, W, _p(gy), L.cout, vchunk, _p(L.dW),
