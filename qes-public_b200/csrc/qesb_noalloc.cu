@@ -353,8 +353,6 @@ extern "C" qesb_status qesb_solve_noalloc(const qesb_grid *grid, float tol, int 
       d.magic = (unsigned)(((1ull << 32) + nq4 - 1) / nq4);
       d.tym = tym;
       d.tzm = tzm;
-      // marks no value of lambda in the buffer can pass for: the bits of negative NaNs, which a solve does not start from
-      d.epoch = 0xffc00000u;
       d.lam = A.lam;
       d.R = A.R;
       d.co = A.co;

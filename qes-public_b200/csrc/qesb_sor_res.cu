@@ -635,6 +635,13 @@ __global__ void __launch_bounds__(kResMaxThreads, 1) k_sor_res(ResArgs a)
       }
     };
     if (D.alias) {
+      // every CTA has read its part of the start: the CTA clears its slots of what lies there (lambda, or an earlier
+      // solve's words, which carry the same marks), before any neighbour asks for them
+      if (tid == 0) meet();
+      __syncthreads();
+      if (s_bad) return;
+      for (int c = 0; c < 2; ++c)
+        for (int i = tid; i < 2 * a.xstride; i += NT) slots(c, rank)[i] = make_ulonglong2(0, 0);
       __syncthreads();
       if (tid == 0) meet();
       __syncthreads();

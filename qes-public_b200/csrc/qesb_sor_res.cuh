@@ -49,7 +49,7 @@ struct ResDomain {
   int nph;
   ResPhase ph[kResPhases];
   ResSync *sync;
-  bool alias;        // lam lies in the exchange buffer (the start is read by all CTAs before the first publishes)
+  bool alias;        // lam lies in the exchange buffer: read by all CTAs, then the slots cleared, before the first publishes
 };
 
 struct ResCtl {

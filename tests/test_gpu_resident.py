@@ -174,3 +174,59 @@ def test_full_coefficients(grid):
     np.testing.assert_array_equal(dev[-1].cpu().numpy(), L)
     for name, t, x in zip("uvw", out, O.correct(d, w, L)):
         np.testing.assert_array_equal(t.cpu().numpy(), x, err_msg=name)
+
+
+def _noalloc(d, w, tol, n, lam0):
+    """One call on the GPU: its stats, lambda and winds."""
+    import torch
+
+    dev = [torch.from_numpy(a).cuda() for a in (*w.inputs(), lam0.copy())]
+    out = [torch.empty(d.numFaceCentered(), device="cuda") for _ in range(3)]
+    torch.cuda.synchronize()
+    st = qesb.solve_noalloc(d, tol, n, *[t.data_ptr() for t in dev], *[t.data_ptr() for t in out])
+    return st, dev[-1].cpu().numpy(), [t.cpu().numpy() for t in out]
+
+
+ROW_GRIDS = [(17, 12, 4), (47, 41, 20), (64, 33, 17), (33, 200, 12), (130, 131, 33)]
+
+
+@pytest.mark.parametrize("grid", ROW_GRIDS)
+def test_no_allocation_calls_of_one_iteration_in_a_row(grid):
+    """The scratch array keeps what the last call left in it: calls of one
+    iteration, each on other inputs than the last, then one of five; every call
+    against the oracle."""
+    ws = [_cut(_city(*grid, seed=s), seed=s) for s in (5, 6)]
+    d = ws[0].domain
+    Rs = [O.divergence(d, w) for w in ws]
+    rng = np.random.default_rng(7)
+    for call, n in enumerate((1, 1, 1, 5, 1, 5)):
+        q = call % 2
+        lam0 = rng.standard_normal(d.numCellCentered()).astype(np.float32)
+        st, lam, winds = _noalloc(d, ws[q], 1e-9, n, lam0)
+        L, it, *_ = O.sor(d, ws[q], Rs[q], 1e-9, n, lam=lam0)
+        assert st["iterations"] == it == n
+        np.testing.assert_array_equal(lam, L)
+        for name, a, x in zip("uvw", winds, O.correct(d, ws[q], L)):
+            np.testing.assert_array_equal(a, x, err_msg=name)
+
+
+@pytest.mark.parametrize("grid", ROW_GRIDS)
+def test_no_allocation_call_that_converges_at_once_then_others(grid):
+    """A coupling loop's quiet step: the kept lambda meets the tolerance in the
+    first iteration; the next steps have other walls and winds."""
+    ws = [_city(*grid, seed=s) for s in (5, 6)]
+    d = ws[0].domain
+    tol, lam = 0.25, np.zeros(d.numCellCentered(), np.float32)
+    its = []
+    for q in (0, 0, 1, 1, 0):
+        w = ws[q]
+        if len(its) == 2:
+            w.u0 *= np.float32(1.5)  # the smallest grids' cities are alike
+        L, it, *_ = O.sor(d, w, O.divergence(d, w), tol, 400, lam=lam)
+        st, lam, winds = _noalloc(d, w, tol, 400, lam)
+        its.append(it)
+        assert st["iterations"] == it and st["converged"] == 1
+        np.testing.assert_array_equal(lam, L)
+        for name, a, x in zip("uvw", winds, O.correct(d, w, L)):
+            np.testing.assert_array_equal(a, x, err_msg=name)
+    assert its[1] == its[3] == 1 < its[2]
