@@ -778,11 +778,12 @@ __global__ void __launch_bounds__(kResMaxThreads, 1) k_sor_res(ResArgs a)
             atomicMax(reinterpret_cast<unsigned long long *>(&s_win), (unsigned long long)__double_as_longlong(dm));
           __syncthreads();
           if (tid == 0) {
-            if (s_win != 0.0) atomic_max_nonneg(&sy->wacc[windows & 1], s_win);
+            const int slot = windows % 3, next = (windows + 1) % 3;
+            if (s_win != 0.0) atomic_max_nonneg(&sy->wacc[slot], s_win);
+            // the next window's slot: its last readers arrived at the barrier before, its next writers leave this one
+            if (rank == 0) *reinterpret_cast<volatile double *>(&sy->wacc[next]) = 0.0;
             meet();
-            s_win = *reinterpret_cast<volatile double *>(&sy->wacc[windows & 1]);
-            // the other slot is next: its last readers arrived at this barrier
-            if (rank == 0) *reinterpret_cast<volatile double *>(&sy->wacc[(windows & 1) ^ 1]) = 0.0;
+            s_win = *reinterpret_cast<volatile double *>(&sy->wacc[slot]);
           }
           __syncthreads();
           if (s_bad) return;

@@ -27,7 +27,7 @@ struct alignas(128) ResSync {
   unsigned long long pad_[14];
   unsigned cert;           // number of the last iteration proven not to stop
   unsigned pad2_;
-  double wacc[2];          // window rule: max|lambda - snapshot|, by window parity
+  double wacc[3];          // window rule: max|lambda - snapshot|, windows in turn
 };
 
 struct ResDomain {

@@ -230,3 +230,21 @@ def test_no_allocation_call_that_converges_at_once_then_others(grid):
         for name, a, x in zip("uvw", winds, O.correct(d, w, L)):
             np.testing.assert_array_equal(a, x, err_msg=name)
     assert its[1] == its[3] == 1 < its[2]
+
+
+@pytest.mark.parametrize("grid", [(17, 12, 4), (47, 41, 20), (130, 131, 33)])
+@pytest.mark.parametrize("K", [1, 2, 3])
+def test_shortest_windows(grid, K):
+    """Windows of one to three iterations, whose maxima follow one another
+    closely: the stop and the last drift are the oracle's, solve after solve."""
+    w = _city(*grid)
+    d = w.domain
+    R = O.divergence(d, w)
+    L = None
+    with qesb.Solver_B200(d, 1e-9) as s:
+        for wtol in (0.05, 0.0125):
+            s.set_window_rule(K, wtol)
+            st = s.solve(w, 2000)
+            L, it, stop, drift = O.sor_window(d, w, R, 1e-9, 2000, K, wtol, lam=L)
+            assert (st["iterations"], st["converged"], st["window_drift"]) == (it, stop, drift) and stop == 2
+            np.testing.assert_array_equal(s.lambda_, L)
