@@ -298,8 +298,9 @@ qesb_status qesb_autotune_batch(qesb_handle *const *handles, int n, int *best, f
  *   "wait_limit"         polls of a staged sweep's shared-memory stage barrier before the kernel gives
  *                        up, lets its copies in flight land, and the solve returns QESB_ERR_CUDA
  *                        ("sweep stage wait gave up"); 0 = the default (2^22 polls). Applies to the
- *                        bulk-copy sweep shapes, the resident kernel's waits for its other CTAs, and
- *                        batches led by this handle */
+ *                        bulk-copy sweep shapes and batches led by this handle, and to each wait of the
+ *                        resident kernel for another tile's half-sweep (default there: 2^23 polls of
+ *                        about a microsecond); it does not bound the length of a solve */
 qesb_status qesb_set_tolerance(qesb_handle *h, float tol);
 qesb_status qesb_set_option(qesb_handle *h, const char *key, int value);
 /* cudaStream_t to run on (NULL = the handle's own stream). */

@@ -328,6 +328,7 @@ extern "C" qesb_status qesb_solve_noalloc(const qesb_grid *grid, float tol, int 
     NaRes A{};
     A.P = 4 * nq4;
     A.CS = (long)A.P * G.Y * G.Z;
+    ctas = nty * ntz;  // a CTA a tile
     const int xstride = 2 * (tym + tzm) * nq4;
     const auto up = [](size_t b) { return (b + 255) / 256 * 256; };
     const size_t xbytes = (size_t)2 * ctas * xstride * 32;

@@ -2099,17 +2099,18 @@ qesb_status res_enqueue(qesb_handle *lead, const std::vector<qesb_handle *> &hs,
   std::memset(L.stage, 0, o_dom);
   // the exchange buffer: room for the largest launch, zeroed when (re)allocated and before its 32-bit marks wrap
   std::vector<ResPlan> plans(n);
-  std::vector<int> xstride(ls.size(), 0);
+  std::vector<int> xstride(ls.size(), 0), gsz(ls.size(), 1);  // no more CTAs a group than a domain has tiles
   size_t xneed = 0;
   unsigned long long halves = 0;
   for (size_t l = 0; l < ls.size(); ++l) {
     for (int q = ls[l].first; q < ls[l].first + ls[l].n; ++q) {
       const qesb_handle *h = hs[order[q]];
       plans[q] = res_plan_of(lead, h->G, ls[l].gsz);
+      gsz[l] = std::max(gsz[l], plans[q].nty * plans[q].ntz);
       xstride[l] = std::max(xstride[l], 2 * (plans[q].tym + plans[q].tzm) * (((h->G.X + 1) / 2 + 3) / 4));
       halves += res_halves(h, itermax);
     }
-    xneed = std::max(xneed, (size_t)ls[l].groups * 2 * ls[l].gsz * xstride[l] * 32);
+    xneed = std::max(xneed, (size_t)ls[l].groups * 2 * gsz[l] * xstride[l] * 32);
   }
   if (L.xbytes < xneed) {
     if (L.xbuf) cudaFree(L.xbuf);
@@ -2182,7 +2183,7 @@ qesb_status res_enqueue(qesb_handle *lead, const std::vector<qesb_handle *> &hs,
     ResArgs a{};
     a.dom = reinterpret_cast<ResDomain *>(L.blk + o_dom) + ls[q].first;
     a.n = ls[q].n;
-    a.gsz = ls[q].gsz;
+    a.gsz = gsz[q];
     a.ctl = reinterpret_cast<ResCtl *>(L.blk) + q;
     a.slot = reinterpret_cast<unsigned long long *>(L.blk + o_slot) + q * sms;
     a.xbuf = reinterpret_cast<ulonglong2 *>(L.xbuf);

@@ -96,6 +96,28 @@ __device__ __forceinline__ bool res_wait(const unsigned long long *p, unsigned l
   return false;
 }
 
+// The same for the group's next domain. A CTA that has no tile of the current
+// one waits here for as long as its solve lasts: the count starts again whenever
+// that solve's iteration number (beat, null before the first domain) has moved.
+__device__ __forceinline__ bool res_wait_next(const unsigned long long *p, unsigned long long want, const unsigned *beat,
+                                              uint32_t limit, ResCtl *ctl)
+{
+  unsigned seen = 0;
+  for (uint32_t n = 0; n < limit; ++n) {
+    if (res_load(p) >= want) return true;
+    if (beat) {
+      const unsigned b = *reinterpret_cast<const volatile unsigned *>(beat);
+      if (b != seen) {
+        seen = b;
+        n = 0;
+      }
+    }
+    if ((n & 1023u) == 1023u && res_fault(ctl)) return false;
+  }
+  atomicExch(&ctl->fault, 1);
+  return false;
+}
+
 __device__ __forceinline__ float max_nan(float a, float b)
 {
   float r;
@@ -397,11 +419,15 @@ __global__ void __launch_bounds__(kResMaxThreads, 1) k_sor_res(ResArgs a)
   __shared__ float s_ctol;
   __shared__ short s_seg[kResSegs + 1];    // the runs' first rows
   __shared__ int s_nw[2];                  // wall cells of each colour
+  __shared__ const unsigned *s_idle;       // the current domain's iteration number, where this CTA has no tile of it
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, NT = blockDim.x, NW = NT >> 5;
   const int rank = blockIdx.x % a.gsz, grp = blockIdx.x / a.gsz;
   const uint32_t limit = a.wait_limit ? a.wait_limit : kResWaitLimit;
   unsigned serial = 0;
-  if (tid == 0) s_bad = 0;
+  if (tid == 0) {
+    s_bad = 0;
+    s_idle = nullptr;
+  }
   for (;;) {
     // the group's next domain
     __syncthreads();
@@ -411,7 +437,7 @@ __global__ void __launch_bounds__(kResMaxThreads, 1) k_sor_res(ResArgs a)
         v = ((unsigned long long)(serial + 1) << 32) | (unsigned)atomicAdd(&a.ctl->queue, 1);
         if (a.gsz > 1) asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(a.slot + grp), "l"(v) : "memory");
       } else {
-        if (!res_wait(a.slot + grp, (unsigned long long)(serial + 1) << 32, limit, a.ctl)) s_bad = 1;
+        if (!res_wait_next(a.slot + grp, (unsigned long long)(serial + 1) << 32, s_idle, limit, a.ctl)) s_bad = 1;
         v = res_load(a.slot + grp);
       }
       s_slot = v;
@@ -425,8 +451,9 @@ __global__ void __launch_bounds__(kResMaxThreads, 1) k_sor_res(ResArgs a)
     if (di >= a.n) return;
     const ResDomain &D = a.dom[di];
     const int nty = D.nty, tiles = nty * D.ntz;
-    if (rank >= tiles) continue;
     ResSync *sy = D.sync;
+    if (tid == 0) s_idle = rank >= tiles ? &sy->beat : nullptr;
+    if (rank >= tiles) continue;
     if (tid == 0) {
       s_target = s_narr = 0;
       t.tym = D.tym;
@@ -749,6 +776,7 @@ __global__ void __launch_bounds__(kResMaxThreads, 1) k_sor_res(ResArgs a)
           const unsigned long long v = s_err[par];
           if (v) atomicMax(reinterpret_cast<unsigned long long *>(F.err + it), v);
           s_err[par] = 0;
+          if (rank == 0) *reinterpret_cast<volatile unsigned *>(&sy->beat) = iters;
           if (!go) {
             meet();
             s_val = *reinterpret_cast<volatile double *>(F.err + it);

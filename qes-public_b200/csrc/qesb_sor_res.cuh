@@ -26,7 +26,7 @@ struct alignas(128) ResSync {
   unsigned long long arr;  // CTAs whose red half-sweep of an iteration is done, summed over the iterations
   unsigned long long pad_[14];
   unsigned cert;           // number of the last iteration proven not to stop
-  unsigned pad2_;
+  unsigned beat;           // the first CTA's iteration number, for CTAs of the group that wait for the next domain
   double wacc[3];          // window rule: max|lambda - snapshot|, windows in turn
 };
 
@@ -61,7 +61,7 @@ struct ResCtl {
 struct ResArgs {
   const ResDomain *dom;
   int n;                     // domains
-  int gsz;                   // CTAs per group
+  int gsz;                   // CTAs per group: the tiles of the launch's most divided domain
   ResCtl *ctl;
   ulonglong2 *xbuf;          // exchange buffer: [group][colour][CTA][xstride] groups of 4 cells, 32 bytes each
   int xstride;

@@ -248,3 +248,29 @@ def test_shortest_windows(grid, K):
             L, it, stop, drift = O.sor_window(d, w, R, 1e-9, 2000, K, wtol, lam=L)
             assert (st["iterations"], st["converged"], st["window_drift"]) == (it, stop, drift) and stop == 2
             np.testing.assert_array_equal(s.lambda_, L)
+
+
+def test_a_wait_limit_bounds_an_exchange_and_not_the_solve():
+    """20000 polls are some ten milliseconds, far more than an exchange takes and
+    far less than the solve: a grid of fewer tiles than the GPU has SMs, alone;
+    then two domains on groups of one size, one of few tiles, each outlasting
+    the limit."""
+    ws = [_city(40, 40, 20), _city(47, 41, 20), _city(17, 12, 4)]
+    n = 12000
+    with qesb.Solver_B200(ws[0].domain, -1.0) as s:
+        s.set_option("wait_limit", 20000)
+        st = s.solve(ws[0], n)
+        assert st["iterations"] == n and st["ms_sor"] > 40.0
+    solvers = [qesb.Solver_B200(w.domain, -1.0) for w in ws[1:]]
+    try:
+        for s, w in zip(solvers, ws[1:]):
+            s.set_inputs(w)
+        solvers[0].set_option("wait_limit", 20000)
+        st = qesb.solve_batch(solvers, n)
+        lam = solvers[1].lambda_
+    finally:
+        for s in solvers:
+            s.close()
+    assert all(x["iterations"] == n and x["ms_sor"] > 30.0 for x in st)
+    w = ws[2]
+    np.testing.assert_array_equal(lam, O.sor(w.domain, w, O.divergence(w.domain, w), -1.0, n)[0])
