@@ -1677,11 +1677,13 @@ qesb_status launch_wgrad(const ConvIn &in, const ConvGeom &g, const __nv_bfloat1
                          int *err, cudaStream_t s)
 {
   constexpr int smem = kWgStages * (128 * 64 * 2 + N * 64 * 2);
-  static bool attr = false;
-  if (!attr) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  static bool attr[64] = {};  // the attribute is a device's own
+  if (!attr[dev & 63]) {
     cudaError_t e = cudaFuncSetAttribute(k_conv_wgrad<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return qesb_fail(QESB_ERR_CUDA, "wgrad attr: %s", cudaGetErrorString(e));
-    attr = true;
+    attr[dev & 63] = true;
   }
   const int cin = in.c1 + in.c2;
   const dim3 grid((unsigned)((27 * cin + 127) / 128), (unsigned)((g.V + vchunk - 1) / vchunk));

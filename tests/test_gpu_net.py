@@ -222,6 +222,30 @@ def test_conv3d_weight_gradient_chunks(D, H, W, ci, co, vchunk, off):
     assert np.all(out[:off] == 0) and np.all(out[off + 27 * ci * co:] == 0)
 
 
+@pytest.mark.parametrize("co", [16, 32, 64, 128])
+def test_conv3d_weight_gradient_on_each_device(co):
+    """Its shared memory is more than a device allows unasked, and each is to be
+    asked: one 64-voxel chunk, so a sum of one CTA's in one order everywhere."""
+    import torch
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two GPUs")
+    torch.manual_seed(co)
+    x, dy = _cl(_bf16(torch.randn(1, 16, 2, 4, 8))), _cl(_bf16(torch.randn(1, co, 2, 4, 8)))
+    out = []
+    for dev in range(2):
+        with torch.cuda.device(dev):
+            dW = torch.zeros(27 * 16 * co, dtype=torch.float32, device="cuda")
+            err = torch.zeros(1, dtype=torch.int32, device="cuda")
+            xd, dyd = x.cuda(), dy.cuda()
+            qesb.check(qesb.lib().qesb_conv3d_wgrad(xd.data_ptr(), 16, 0, None, 0, 2, 4, 8, dyd.data_ptr(), co, 64,
+                                                    dW.data_ptr(), err.data_ptr(), None))
+            torch.cuda.synchronize()
+            assert int(err.item()) == 0
+            out.append(dW.cpu().numpy())
+    assert np.any(out[0] != 0)
+    np.testing.assert_array_equal(out[0], out[1])
+
+
 # ---------------------------------------------------------------------------
 # direct conv3d kernel (rows of 128 voxels): same contract as the implicit GEMM
 # ---------------------------------------------------------------------------
