@@ -41,6 +41,7 @@
 #include "qesb_sor_tiled.cuh"
 #include "qesb_sor_split.cuh"
 #include "qesb_sor_zm.cuh"
+#include "qesb_res_plan.h"
 #include "qesb_sor_res.cuh"
 #include "qesb_wall_log.cuh"
 #include "qesb_fp64.cuh"
@@ -838,14 +839,6 @@ struct SweepGraph {
   }
 };
 
-// Tiles of a resident solve (qesb_sor_res.cu) over at most so many CTAs, with the
-// estimated cycles of a half-sweep; nty = 0: the domain does not fit.
-struct ResPlan {
-  int nty = 0, ntz = 0;
-  int tym = 0, tzm = 0;  // the largest tile
-  double cost = 0;
-};
-
 struct qesb_handle {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -960,7 +953,7 @@ struct qesb_handle {
     unsigned char *xbuf = nullptr;
     size_t xbytes = 0;
     unsigned long long epoch = 0;
-    std::map<std::tuple<int, int, int, int>, ResPlan> plans;  // by grid and CTAs
+    ResPlans plans;
   } rlist;
 
   // iteration-loop graphs of the tiled path, one per (variant, starting buffer)
@@ -1119,7 +1112,7 @@ qesb_status ensure_split_coefs(qesb_handle *h)
   return QESB_OK;
 }
 
-const ResPlan &res_plan_of(qesb_handle *lead, const DevGrid &G, int ctas);
+ResPlan res_plan_of(qesb_handle *lead, const DevGrid &G, int ctas);
 int res_ctas(int device);
 
 // R for a solve: the R already computed from the same inputs (a warm start
@@ -1810,10 +1803,6 @@ qesb_status run_iterations_sweep(qesb_handle *h, const SweepVariant &sv, int ite
 // ---------------------------------------------------------------------------
 // resident solves (qesb_sor_res.cuh)
 // ---------------------------------------------------------------------------
-constexpr int kResThreads = 512;         // one CTA per SM
-constexpr int kResSmemBytes = 230400;    // the per-block limit less the kernel's static part
-constexpr int kResMaxLaunches = 16;           // launches of one batch (group sizes)
-
 __global__ void k_res_stamp(ResCtl *ctl) { ctl->t0 = global_ns(); }
 
 // lambda and R of the padded layout into the split layout, one pass.
@@ -1842,40 +1831,6 @@ __global__ void k_res_to_pad(DevGrid G, SplitGeom S, const float *__restrict__ s
     dst[G.pad(i, j, k)] = src[((i + j + ks) & 1) * S.CS + S.row(j, ks, G.Y) + (i >> 1)];
 }
 
-// The estimate: row steps of the CTA's warps (350 cycles for all of them, dearer
-// where R streams from L2) and the exchange. Measured solves take 1.45 (the
-// smallest domains) to 1.95 times it: 1.85, at 1.9 GHz, in kResUs.
-constexpr double kResUs = 2 * 1.85 / 1900.0;  // microseconds an iteration per estimated cycle of a half-sweep
-ResPlan res_plan(const DevGrid &G, int ctas)
-{
-  constexpr int NW = kResThreads / 32;
-  ResPlan best;
-  const int nq4 = ((G.X + 1) / 2 + 3) / 4, P = 4 * nq4, rows = G.Y - 2, planes = G.Z - 2;
-  const long cap = kResSmemBytes / 4;
-  // for each cut along z the most tiles along y that the CTAs allow (no more than their row count needs)
-  for (int ntz = 1; ntz <= std::min(planes, ctas); ++ntz) {
-    const int tz = (planes + ntz - 1) / ntz, ty = (rows + std::min(rows, ctas / ntz) - 1) / std::min(rows, ctas / ntz);
-    const int nty = (rows + ty - 1) / ty;
-    const long base = 2048 + 72L * tz + 2L * (tz + 2) * (ty + 2) * P + 2L * tz * ty * nq4 + 4L * (tz + ty) * nq4 + 8;
-    if (base > cap) continue;
-    const int rp = (int)std::min<long>(tz, (cap - base) / (2L * ty * P));
-    const int ch = ((tz + 1) / 2 * nq4 + 31) / 32 + (tz / 2 * nq4 + 31) / 32;  // warps' columns
-    int steps = 1 << 30;
-    for (int n = 1; n <= std::min(ty, 32); ++n) steps = std::min(steps, (ch * n + NW - 1) / NW * ((ty + n - 1) / n + 4));
-    const double step = 350.0 * (1.0 + 0.4 * (tz - rp) / tz);
-    const double comm = nty * ntz > 1 ? 2000.0 + 0.25 * (tz + ty) * nq4 : 200.0;
-    const double cost = step * steps + comm;
-    if (best.nty == 0 || cost < best.cost) {
-      best.nty = nty;
-      best.ntz = ntz;
-      best.cost = cost;
-      best.tym = ty;
-      best.tzm = tz;
-    }
-  }
-  return best;
-}
-
 int sm_count(int device)
 {
   static int nsm[64] = {};
@@ -1895,17 +1850,8 @@ unsigned long long res_halves(const qesb_handle *h, int itermax)
   return 2ull * ((unsigned long long)itermax + (prephase_on(h) ? h->pre_iters : 0) + (start_on(h) ? h->start_iters : 0) + 1);
 }
 
-const ResPlan &res_plan_of(qesb_handle *lead, const DevGrid &G, int ctas)
-{
-  auto &m = lead->rlist.plans;
-  const std::tuple<int, int, int, int> key(G.X, G.Y, G.Z, ctas);
-  auto it = m.find(key);
-  if (it == m.end()) {
-    if (m.size() > 4096) m.clear();
-    it = m.emplace(key, res_plan(G, ctas)).first;
-  }
-  return it->second;
-}
+ResSize res_size(const DevGrid &G) { return {G.X, G.Y, G.Z}; }
+ResPlan res_plan_of(qesb_handle *lead, const DevGrid &G, int ctas) { return lead->rlist.plans.of(res_size(G), ctas); }
 
 // Whether a solve of h led by `lead` may take the resident kernel: no sweep
 // shape asked for, lambda fits the chip's shared memory, and the half-sweeps it
@@ -1924,138 +1870,6 @@ bool res_may(qesb_handle *lead, const qesb_handle *h, int itermax, unsigned long
   return true;
 }
 
-// The launches of a list of domains: domains of about the same best group size
-// go together, large ones first.
-struct ResLaunch {
-  int first, n, groups, gsz;  // of `order`
-};
-struct ResSchedule {
-  std::vector<int> order;
-  std::vector<ResLaunch> launches;
-  double cost = 0;           // estimated cycles of a half-sweep of all domains
-  std::vector<double> each;  // a domain's own share of it
-};
-ResSchedule res_schedule(qesb_handle *lead, const std::vector<qesb_handle *> &hs)
-{
-  const int n = (int)hs.size(), sms = res_ctas(lead->device);
-  ResSchedule r;
-  r.order.resize(n);
-  r.each.resize(n);
-  std::vector<int> ng(n);
-  for (int i = 0; i < n; ++i) {
-    r.order[i] = i;
-    for (int g = 1; g <= std::min(n, sms); ++g) {
-      const ResPlan &p = res_plan_of(lead, hs[i]->G, sms / g);
-      if (!p.nty) break;
-      if (ng[i] == 0 || p.cost / g < r.each[i]) {
-        r.each[i] = p.cost / g;
-        ng[i] = g;
-      }
-    }
-  }
-  std::stable_sort(r.order.begin(), r.order.end(), [&](int a, int b) {
-    if (ng[a] != ng[b]) return ng[a] < ng[b];
-    return hs[a]->G.XY * hs[a]->G.Z > hs[b]->G.XY * hs[b]->G.Z;
-  });
-  // the time of one launch of order[i, j) in g groups: each takes the next domain when it is free
-  auto span = [&](int i, int j, int g) {
-    std::vector<double> t(g, 0.0);
-    for (int q = i; q < j; ++q) {
-      const ResPlan &p = res_plan_of(lead, hs[r.order[q]]->G, sms / g);
-      if (!p.nty) return -1.0;
-      *std::min_element(t.begin(), t.end()) += p.cost;
-    }
-    return *std::max_element(t.begin(), t.end());
-  };
-  auto best_launch = [&](int i, int j, double *cost) {
-    ResLaunch l{i, j - i, 1, sms};
-    *cost = span(i, j, 1);
-    for (int g = 2; g <= std::min(j - i, sms); ++g) {
-      const double c = span(i, j, g);
-      if (c < 0) break;
-      if (c < *cost) {
-        *cost = c;
-        l.groups = g;
-        l.gsz = sms / g;
-      }
-    }
-    return l;
-  };
-  for (int i = 0; i < n;) {
-    int j = i;
-    while (j < n && ng[r.order[j]] == ng[r.order[i]]) ++j;
-    double c = 0;
-    ResLaunch l = best_launch(i, j, &c);
-    if (!r.launches.empty()) {  // together with the launch before where that is shorter (or there are many)
-      const ResLaunch &b = r.launches.back();
-      double cb = 0, cm = 0;
-      const ResLaunch before = best_launch(b.first, i, &cb), m = best_launch(b.first, j, &cm);
-      (void)before;
-      if (cm <= cb + c || (int)r.launches.size() == kResMaxLaunches) {
-        r.launches.back() = m;
-        r.cost += cm - cb;
-        i = j;
-        continue;
-      }
-    }
-    r.launches.push_back(l);
-    r.cost += c;
-    i = j;
-  }
-  return r;
-}
-
-// Microseconds that a domain adds to an iteration of the streaming list sweeps
-// (measured: 3.0 a million cells on full 128-cell row tiles, 4.5 where half of a
-// tile is empty), and what the list's launches take of themselves.
-double list_us(const DevGrid &G)
-{
-  const int qn = (G.X + 1) / 2;
-  return 3.0e-6 * (double)G.XY * G.Z * 0.5 * (1.0 + 128.0 * ((qn + 127) / 128) / qn);
-}
-constexpr double kListUs = 12.0;
-
-// Which domains of a batch take the resident kernel, of those that may: all,
-// none, or those it is faster for than their part of the list sweeps, by the
-// shorter estimate. A list of small domains gains the most (16 of 64 x 64 x 32:
-// 10 against 35 us an iteration; 16 of 128 x 128 x 48: 42 against 76), many
-// large ones (16 of 192 x 192 x 64: 171 against 133) stay with the list sweeps.
-std::vector<char> res_choose(qesb_handle *lead, qesb_handle *const *hs, int n, const std::vector<char> &may)
-{
-  std::vector<qesb_handle *> all;
-  std::vector<int> of;
-  double others = 0;  // list time of the domains that have no choice
-  for (int i = 0; i < n; ++i) {
-    if (may[i]) {
-      all.push_back(hs[i]);
-      of.push_back(i);
-    } else {
-      others += list_us(hs[i]->G);
-    }
-  }
-  std::vector<char> none(n, 0);
-  if (all.empty()) return none;
-  const ResSchedule sch = res_schedule(lead, all);
-  double list_all = 0, list_rest = 0;
-  std::vector<char> some(n, 0);
-  std::vector<qesb_handle *> part;
-  for (size_t q = 0; q < all.size(); ++q) {
-    const double l = list_us(all[q]->G);
-    list_all += l;
-    if (kResUs * sch.each[q] < l) {
-      some[of[q]] = 1;
-      part.push_back(all[q]);
-    } else {
-      list_rest += l;
-    }
-  }
-  const auto list = [&](double us) { return us + others > 0 ? us + others + kListUs : 0.0; };
-  const double t_all = kResUs * sch.cost + list(0.0), t_none = list(list_all);
-  const double t_some = part.empty() ? t_none : kResUs * res_schedule(lead, part).cost + list(list_rest);
-  if (t_none <= t_all && t_none <= t_some) return none;
-  return t_all <= t_some ? may : some;
-}
-
 qesb_status res_prepare(qesb_handle *h)
 {
   const int need = (prephase_on(h) ? h->pre_iters : 0) + (start_on(h) ? h->start_iters : 0);
@@ -2070,16 +1884,15 @@ qesb_status res_prepare(qesb_handle *h)
 }
 
 // Solves the handles' domains (R computed, err and state zeroed on s) from their current lambda to the end of their reference loops:
-// one cooperative launch per group size. Enqueues everything on s, the final
+// the launches of `sch`, cooperative ones. Enqueues everything on s, the final
 // states' copies to the mapped buffers included; the caller waits and then
 // calls res_finish. full: with each cell's own coefficients (d_cs), the
 // reference loop alone. *launches: kernels launched.
-qesb_status res_enqueue(qesb_handle *lead, const std::vector<qesb_handle *> &hs, bool full, int itermax, cudaStream_t s,
-                        int *launches)
+qesb_status res_enqueue(qesb_handle *lead, const std::vector<qesb_handle *> &hs, const ResSchedule &sch, bool full,
+                        int itermax, cudaStream_t s, int *launches)
 {
   const int n = (int)hs.size(), sms = res_ctas(lead->device);
   WordBatch wb(s);
-  const ResSchedule sch = res_schedule(lead, hs);
   const std::vector<int> &order = sch.order;
   const std::vector<ResLaunch> &ls = sch.launches;
   // descriptors: [launch controls][group slots][domains]
@@ -2235,7 +2048,8 @@ qesb_status run_iterations_resident(qesb_handle *h, bool full, int itermax)
   cudaStream_t s = h->stream;
   CKS(res_prepare(h));
   if (full) CKS(ensure_split_coefs(h));
-  CKS(res_enqueue(h, {h}, full, itermax, s, &h->last_launches));
+  CKS(res_enqueue(h, {h}, res_schedule(h->rlist.plans, {res_size(h->G)}, res_ctas(h->device)), full, itermax, s,
+                  &h->last_launches));
   for (int q = 2; q < 4; ++q) CK(cudaEventRecord(h->evs[q], s));  // one launch runs every phase: evs[0..1]
   h->sweeps_timed = !full;
   return QESB_OK;
@@ -3011,9 +2825,14 @@ qesb_status qesb_solve_batch(qesb_handle *const *hs, int n, int itermax, float *
   std::vector<qesb_handle *> res;
   std::vector<int> res_of, str_of;  // batch indices
   unsigned long long room = kResMarks;
-  std::vector<char> is_res(n, 0);
-  for (int i = 0; i < n; ++i) is_res[i] = res_may(h0, hs[i], itermax, &room);
-  is_res = res_choose(h0, hs, n, is_res);
+  std::vector<char> may(n, 0);
+  std::vector<ResSize> sizes;
+  for (int i = 0; i < n; ++i) {
+    may[i] = res_may(h0, hs[i], itermax, &room);
+    sizes.push_back(res_size(hs[i]->G));
+  }
+  const ResChoice choice = res_choose(h0->rlist.plans, sizes, may, res_ctas(h0->device));
+  const std::vector<char> &is_res = choice.is_res;
   for (int i = 0; i < n; ++i) {
     if (is_res[i]) {
       res.push_back(hs[i]);
@@ -3071,7 +2890,7 @@ qesb_status qesb_solve_batch(qesb_handle *const *hs, int n, int itermax, float *
   float ms_res = 0;
   unsigned long long t0_res = 0;
   if (!res.empty()) {
-    CKS(res_enqueue(h0, res, false, itermax, s, &res_launches));
+    CKS(res_enqueue(h0, res, choice.sched, false, itermax, s, &res_launches));
     if (!doms.empty()) {  // the list sweeps reuse the events
       CK(cudaStreamSynchronize(s));
       CK(cudaEventElapsedTime(&ms_res, h0->evs[0], h0->evs[1]));
@@ -3241,12 +3060,8 @@ qesb_status qesb_set_prephase(qesb_handle *h, float omega, float tol, int max_it
 void qesb_res_tiles(int X, int Y, int Z, int device, int *nty, int *ntz, int *tym, int *tzm, int *ctas, int *threads,
                     int *smem_floats)
 {
-  DevGrid G{};
-  G.X = X;
-  G.Y = Y;
-  G.Z = Z;
   *ctas = res_ctas(device);
-  const ResPlan p = res_plan(G, *ctas);
+  const ResPlan p = res_plan({X, Y, Z}, *ctas);
   *nty = p.nty;
   *ntz = p.ntz;
   *tym = p.tym;
