@@ -273,12 +273,14 @@ qesb_status qesb_workspace_read(const char *path, int Nx, int Ny, int Nz, float 
                                 float *w0, float *u, float *v, float *w);
 
 /* Batch autotuner: times every sweep launch shape on the domain list that
- * qesb_solve_batch would run for these handles (same checks), a few launches
- * each from the handles' current lambda, and stores the fastest as
- * handles[0]'s "batch_variant" option, which qesb_solve_batch then uses.
+ * qesb_solve_batch would run for these handles (same checks): the domains that
+ * it does not solve with lambda resident in shared memory (option "variant"),
+ * or all of them where it would solve every one that way. A few launches each
+ * from the handles' current lambda; the fastest is stored as handles[0]'s
+ * "batch_variant" option, which qesb_solve_batch then uses for its list.
  * lambda is left unchanged (the sweeps advance the split-layout copy only).
  * us_per_iter (nullable, n_variants entries) receives each shape's time per
- * iteration over the whole list, at its variant index (entries below the
+ * iteration over that list, at its variant index (entries below the
  * first sweep shape are left untouched); *best the chosen index. */
 qesb_status qesb_autotune_batch(qesb_handle *const *handles, int n, int *best, float *us_per_iter, int n_variants);
 
@@ -292,8 +294,10 @@ qesb_status qesb_autotune_batch(qesb_handle *const *handles, int n, int *best, f
  *   "variant"            sweep variant index, see qesb_num_variants (-1 = the solver's choice: a domain whose
  *                        lambda fits the chip's shared memory, up to about 5 million cells, is solved by one
  *                        cooperative launch with lambda resident there; others run the autotuned / default shape)
- *   "batch_variant"      sweep shape for qesb_solve_batch led by this handle (-1 = from "variant");
- *                        set by qesb_autotune_batch
+ *   "batch_variant"      shape of the list sweeps of qesb_solve_batch led by this handle (-1 = from "variant");
+ *                        set by qesb_autotune_batch. It shapes the list only: domains that are faster
+ *                        with lambda resident are solved that way all the same. "variant" on
+ *                        handles[0] names a shape for every domain of the batch
  *   "autotune"           1 = run qesb_autotune at the first solve of an untuned grid shape (default 0)
  *   "wait_limit"         polls of a staged sweep's shared-memory stage barrier before the kernel gives
  *                        up, lets its copies in flight land, and the solve returns QESB_ERR_CUDA

@@ -1870,6 +1870,18 @@ bool res_may(qesb_handle *lead, const qesb_handle *h, int itermax, unsigned long
   return true;
 }
 
+ResChoice batch_choice(qesb_handle *lead, qesb_handle *const *hs, int n, int itermax)
+{
+  unsigned long long room = kResMarks;
+  std::vector<char> may(n, 0);
+  std::vector<ResSize> sizes;
+  for (int i = 0; i < n; ++i) {
+    may[i] = res_may(lead, hs[i], itermax, &room);
+    sizes.push_back(res_size(hs[i]->G));
+  }
+  return res_choose(lead->rlist.plans, sizes, may, res_ctas(lead->device));
+}
+
 qesb_status res_prepare(qesb_handle *h)
 {
   const int need = (prephase_on(h) ? h->pre_iters : 0) + (start_on(h) ? h->start_iters : 0);
@@ -2727,12 +2739,19 @@ static qesb_status batch_check(qesb_handle *const *hs, int n, const char *who)
   return QESB_OK;
 }
 
-qesb_status qesb_autotune_batch(qesb_handle *const *hs, int n, int *best, float *us_per_iter, int n_variants)
+qesb_status qesb_autotune_batch(qesb_handle *const *handles, int n_handles, int *best, float *us_per_iter, int n_variants)
 {
-  CKS(batch_check(hs, n, "qesb_autotune_batch"));
-  qesb_handle *h0 = hs[0];
+  CKS(batch_check(handles, n_handles, "qesb_autotune_batch"));
+  qesb_handle *h0 = handles[0];
   CK(cudaSetDevice(h0->device));
   cudaStream_t s = h0->stream;
+  // the domains that a batch solve leaves to the list sweeps, or all where it leaves none
+  const ResChoice choice = batch_choice(h0, handles, n_handles, 1);
+  std::vector<qesb_handle *> hs;
+  for (int i = 0; i < n_handles; ++i)
+    if (!choice.is_res[i]) hs.push_back(handles[i]);
+  if (hs.empty()) hs.assign(handles, handles + n_handles);
+  const int n = (int)hs.size();
   // the domains as a solve would start them: R, and lambda and R in the split
   // layout (the tuning sweeps advance only the split copy; a solve re-derives
   // it from lambda)
@@ -2824,14 +2843,7 @@ qesb_status qesb_solve_batch(qesb_handle *const *hs, int n, int itermax, float *
   // domains solved by the resident kernel, and by the list sweeps
   std::vector<qesb_handle *> res;
   std::vector<int> res_of, str_of;  // batch indices
-  unsigned long long room = kResMarks;
-  std::vector<char> may(n, 0);
-  std::vector<ResSize> sizes;
-  for (int i = 0; i < n; ++i) {
-    may[i] = res_may(h0, hs[i], itermax, &room);
-    sizes.push_back(res_size(hs[i]->G));
-  }
-  const ResChoice choice = res_choose(h0->rlist.plans, sizes, may, res_ctas(h0->device));
+  const ResChoice choice = batch_choice(h0, hs, n, itermax);
   const std::vector<char> &is_res = choice.is_res;
   for (int i = 0; i < n; ++i) {
     if (is_res[i]) {

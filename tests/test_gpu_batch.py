@@ -232,3 +232,37 @@ def test_flags_only_inputs_give_the_same_solve():
         assert a[0] == b[0] and a[1] == b[1]
         for x, y in zip(a[2:], b[2:]):
             np.testing.assert_array_equal(x, y)
+
+
+def test_batch_autotune_times_the_list_that_runs():
+    """One domain too large for shared memory among twelve that are solved with
+    lambda resident there: the tuner times the large one's sweeps, as for it
+    alone, and not the thirteen's, which take more than twice as long."""
+    dims = [(300, 300, 50)] + [(128, 128, 48)] * 12
+    ws = []
+    for q, (nx, ny, nz) in enumerate(dims[:2]):
+        d = qesb.Domain(nx, ny, nz, 2.0, 2.0, 1.0, qesb.city_dz(nz, 1.0, 1.03))
+        c = qesb.city_random(d, 7 + q, 12, fp=(6, 20), h=(4, 20))
+        ws.append(qesb.city_build(d, c.buildings, c.inflow))
+    ws += [ws[1]] * 11
+    solvers = [qesb.Solver_B200(w.domain, 1e-9) for w in ws]
+    try:
+        for s, w in zip(solvers, ws):
+            s.set_inputs(w)
+        best = {}
+        for who, lst in (("alone", solvers[:1]), ("mixed", solvers)):
+            b, us = qesb.autotune_batch(lst)
+            best[who] = us[b]
+        solvers[0].set_option("variant", 18)  # a shape for every domain: the list is the whole batch
+        b, us = qesb.autotune_batch(solvers)
+        best["all"] = us[b]
+        solvers[0].set_option("variant", -1)
+        st = qesb.solve_batch(solvers, 5)
+        lam = solvers[0].lambda_, solvers[5].lambda_
+    finally:
+        for s in solvers:
+            s.close()
+    assert best["all"] > 2 * best["alone"] and best["mixed"] < 1.5 * best["alone"], best
+    assert all(x["iterations"] == 5 for x in st)
+    for L, w in zip(lam, ws):
+        np.testing.assert_array_equal(L, O.sor(w.domain, w, O.divergence(w.domain, w), 1e-9, 5)[0])
