@@ -1079,6 +1079,15 @@ qesb_status ensure_padded_coefs(qesb_handle *h)
   return QESB_OK;
 }
 
+// Device memory that a faster way needs and a slower one does without.
+bool try_alloc(void **p, size_t bytes)
+{
+  if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+  cudaGetLastError();
+  *p = nullptr;
+  return false;
+}
+
 // The coefficients in the split layout, and omega / (their sum) (the division
 // of every update, Solver_CPU_RB.cpp:118, done once).
 __global__ void k_split_coefs(DevGrid G, SplitGeom S, const float *__restrict__ e, const float *__restrict__ f,
@@ -1100,11 +1109,12 @@ __global__ void k_split_coefs(DevGrid G, SplitGeom S, const float *__restrict__ 
   }
 }
 
+// Sets cs_ready, unless the device has no room for the copies.
 qesb_status ensure_split_coefs(qesb_handle *h)
 {
   if (h->cs_ready) return QESB_OK;
   const DevGrid &G = h->G;
-  if (!h->d_cs) CKS(dalloc(&h->d_cs, 14 * (size_t)h->S.CS));
+  if (!h->d_cs && !try_alloc((void **)&h->d_cs, 14 * (size_t)h->S.CS * sizeof(float))) return QESB_OK;
   k_split_coefs<<<row_grid(G, G.Y, G.Z, G.X), 256, 0, h->stream>>>(G, h->S, h->d_in[0], h->d_in[1], h->d_in[2], h->d_in[3],
                                                                   h->d_in[4], h->d_in[5], h->d_cs);
   CK(cudaGetLastError());
@@ -1156,7 +1166,8 @@ qesb_status prepare_coefs(qesb_handle *h)
   // it is the only path, else at its first use.
   h->pc_ready = false;
   h->cs_ready = false;
-  if (!h->packed) CKS(res_plan_of(h, G, res_ctas(h->device)).nty > 0 ? ensure_split_coefs(h) : ensure_padded_coefs(h));
+  if (!h->packed && res_plan_of(h, G, res_ctas(h->device)).nty > 0) CKS(ensure_split_coefs(h));
+  if (!h->packed && !h->cs_ready) CKS(ensure_padded_coefs(h));
   return QESB_OK;
 }
 
@@ -1895,11 +1906,70 @@ qesb_status res_prepare(qesb_handle *h)
   return QESB_OK;
 }
 
+// What the launches of a schedule need, beyond the domains' own.
+struct ResLayout {
+  std::vector<ResPlan> plans;    // by place in the order
+  std::vector<int> xstride, gsz; // by launch; no more CTAs a group than a domain has tiles
+  size_t xbytes = 0;             // the tiles' exchange buffer: room for the largest launch
+};
+ResLayout res_layout(qesb_handle *lead, const std::vector<ResSize> &ds, const ResSchedule &sch)
+{
+  ResLayout r;
+  r.plans.resize(ds.size());
+  for (const ResLaunch &l : sch.launches) {
+    int xs = 0, gsz = 1;
+    for (int q = l.first; q < l.first + l.n; ++q) {
+      const ResSize &d = ds[sch.order[q]];
+      const ResPlan p = r.plans[q] = lead->rlist.plans.of(d, l.gsz);
+      xs = std::max(xs, 2 * (p.tym + p.tzm) * (((d.X + 1) / 2 + 3) / 4));
+      gsz = std::max(gsz, p.nty * p.ntz);
+    }
+    r.xstride.push_back(xs);
+    r.gsz.push_back(gsz);
+    r.xbytes = std::max(r.xbytes, (size_t)l.groups * 2 * gsz * xs * 32);
+  }
+  return r;
+}
+
+// Descriptors in device memory: [launch controls][group slots][domains]
+size_t res_dom_offset(int sms) { return (sizeof(ResCtl) + sizeof(unsigned long long) * (size_t)sms) * kResMaxLaunches; }
+
+// Makes room on lead for a launch of these domains (nothing where there is
+// enough; a handle has it for its own domain from its creation). False: the
+// device has none, and the solves take the sweeps.
+bool res_reserve(qesb_handle *lead, const std::vector<ResSize> &ds, const ResSchedule &sch)
+{
+  const int n = (int)ds.size();
+  const size_t xbytes = res_layout(lead, ds, sch).xbytes;
+  qesb_handle::ResList &L = lead->rlist;
+  if (L.cap < n) {
+    if (L.blk) cudaFree(L.blk);
+    if (L.stage) cudaFreeHost(L.stage);
+    L.blk = L.stage = nullptr;
+    L.cap = 0;
+    const size_t bytes = res_dom_offset(res_ctas(lead->device)) + sizeof(ResDomain) * (size_t)n;
+    if (!try_alloc((void **)&L.blk, bytes) || host_mapped(&L.stage, &L.stage_dev, bytes) != QESB_OK) {
+      cudaGetLastError();
+      return false;
+    }
+    L.cap = n;
+  }
+  if (L.xbytes < xbytes) {
+    if (L.xbuf) cudaFree(L.xbuf);
+    L.xbuf = nullptr;
+    L.xbytes = 0;
+    L.epoch = ~0ull;
+    if (!try_alloc((void **)&L.xbuf, xbytes)) return false;
+    L.xbytes = xbytes;
+  }
+  return true;
+}
+
 // Solves the handles' domains (R computed, err and state zeroed on s) from their current lambda to the end of their reference loops:
 // the launches of `sch`, cooperative ones. Enqueues everything on s, the final
 // states' copies to the mapped buffers included; the caller waits and then
 // calls res_finish. full: with each cell's own coefficients (d_cs), the
-// reference loop alone. *launches: kernels launched.
+// reference loop alone. Room is reserved. *launches: kernels launched.
 qesb_status res_enqueue(qesb_handle *lead, const std::vector<qesb_handle *> &hs, const ResSchedule &sch, bool full,
                         int itermax, cudaStream_t s, int *launches)
 {
@@ -1907,44 +1977,17 @@ qesb_status res_enqueue(qesb_handle *lead, const std::vector<qesb_handle *> &hs,
   WordBatch wb(s);
   const std::vector<int> &order = sch.order;
   const std::vector<ResLaunch> &ls = sch.launches;
-  // descriptors: [launch controls][group slots][domains]
-  const size_t o_slot = sizeof(ResCtl) * kResMaxLaunches,
-               o_dom = o_slot + sizeof(unsigned long long) * (size_t)kResMaxLaunches * sms;
+  const size_t o_slot = sizeof(ResCtl) * kResMaxLaunches, o_dom = res_dom_offset(sms);
   qesb_handle::ResList &L = lead->rlist;
-  if (L.cap < n) {
-    if (L.blk) cudaFree(L.blk);
-    if (L.stage) cudaFreeHost(L.stage);
-    L.blk = L.stage = nullptr;
-    L.cap = 0;
-    const size_t bytes = o_dom + sizeof(ResDomain) * (size_t)n;
-    CK(cudaMalloc((void **)&L.blk, bytes));
-    CKS(host_mapped(&L.stage, &L.stage_dev, bytes));
-    L.cap = n;
-  }
   std::memset(L.stage, 0, o_dom);
-  // the exchange buffer: room for the largest launch, zeroed when (re)allocated and before its 32-bit marks wrap
-  std::vector<ResPlan> plans(n);
-  std::vector<int> xstride(ls.size(), 0), gsz(ls.size(), 1);  // no more CTAs a group than a domain has tiles
-  size_t xneed = 0;
+  std::vector<ResSize> ds;
   unsigned long long halves = 0;
-  for (size_t l = 0; l < ls.size(); ++l) {
-    for (int q = ls[l].first; q < ls[l].first + ls[l].n; ++q) {
-      const qesb_handle *h = hs[order[q]];
-      plans[q] = res_plan_of(lead, h->G, ls[l].gsz);
-      gsz[l] = std::max(gsz[l], plans[q].nty * plans[q].ntz);
-      xstride[l] = std::max(xstride[l], 2 * (plans[q].tym + plans[q].tzm) * (((h->G.X + 1) / 2 + 3) / 4));
-      halves += res_halves(h, itermax);
-    }
-    xneed = std::max(xneed, (size_t)ls[l].groups * 2 * gsz[l] * xstride[l] * 32);
+  for (const qesb_handle *h : hs) {
+    ds.push_back(res_size(h->G));
+    halves += res_halves(h, itermax);
   }
-  if (L.xbytes < xneed) {
-    if (L.xbuf) cudaFree(L.xbuf);
-    L.xbuf = nullptr;
-    L.xbytes = 0;
-    CK(cudaMalloc((void **)&L.xbuf, xneed));
-    L.xbytes = xneed;
-    L.epoch = ~0ull;
-  }
+  const ResLayout lay = res_layout(lead, ds, sch);
+  // zeroed when (re)allocated and before its 32-bit marks wrap
   if (L.epoch == ~0ull || L.epoch + halves >= 0xffffff00ull) {
     CK(zero_async(L.xbuf, L.xbytes, s));
     L.epoch = 0;
@@ -1954,7 +1997,7 @@ qesb_status res_enqueue(qesb_handle *lead, const std::vector<qesb_handle *> &hs,
     for (int q = l.first; q < l.first + l.n; ++q) {
       qesb_handle *h = hs[order[q]];
       const DevGrid &G = h->G;
-      const ResPlan &p = plans[q];
+      const ResPlan &p = lay.plans[q];
       ResDomain d{};
       d.X = G.X;
       d.Y = G.Y;
@@ -2008,11 +2051,11 @@ qesb_status res_enqueue(qesb_handle *lead, const std::vector<qesb_handle *> &hs,
     ResArgs a{};
     a.dom = reinterpret_cast<ResDomain *>(L.blk + o_dom) + ls[q].first;
     a.n = ls[q].n;
-    a.gsz = gsz[q];
+    a.gsz = lay.gsz[q];
     a.ctl = reinterpret_cast<ResCtl *>(L.blk) + q;
     a.slot = reinterpret_cast<unsigned long long *>(L.blk + o_slot) + q * sms;
     a.xbuf = reinterpret_cast<ulonglong2 *>(L.xbuf);
-    a.xstride = xstride[q];
+    a.xstride = lay.xstride[q];
     a.wait_limit = lead->opt_wait_limit;
     a.smem_floats = kResSmemBytes / 4;
     CK(res_launch(a, full, ls[q].groups, kResThreads, s));
@@ -2055,13 +2098,11 @@ qesb_status res_finish(qesb_handle *lead, const std::vector<qesb_handle *> &hs, 
 }
 
 // One solve on the resident kernel: as run_iterations_sweep, in one launch.
-qesb_status run_iterations_resident(qesb_handle *h, bool full, int itermax)
+qesb_status run_iterations_resident(qesb_handle *h, const ResSchedule &sch, bool full, int itermax)
 {
   cudaStream_t s = h->stream;
   CKS(res_prepare(h));
-  if (full) CKS(ensure_split_coefs(h));
-  CKS(res_enqueue(h, {h}, res_schedule(h->rlist.plans, {res_size(h->G)}, res_ctas(h->device)), full, itermax, s,
-                  &h->last_launches));
+  CKS(res_enqueue(h, {h}, sch, full, itermax, s, &h->last_launches));
   for (int q = 2; q < 4; ++q) CK(cudaEventRecord(h->evs[q], s));  // one launch runs every phase: evs[0..1]
   h->sweeps_timed = !full;
   return QESB_OK;
@@ -2099,7 +2140,16 @@ qesb_status solve_impl(qesb_handle *h, int itermax, float *u, float *v, float *w
   CK(cudaEventRecord(h->ev[1], s));
   const bool packed = h->packed && h->opt_path == 1;
   unsigned long long room = kResMarks;
-  const bool resident = res_may(h, h, itermax, &room);
+  bool resident = res_may(h, h, itermax, &room);
+  ResSchedule sch;
+  if (resident) {
+    sch = res_schedule(h->rlist.plans, {res_size(G)}, res_ctas(h->device));
+    resident = res_reserve(h, {res_size(G)}, sch);
+  }
+  if (resident && !packed) {
+    CKS(ensure_split_coefs(h));
+    resident = h->cs_ready;
+  }
   if (packed && !resident && h->opt_autotune && h->opt_variant < 0 && tuned_variant(G) < 0) {
     CKS(qesb_autotune(h, nullptr, nullptr, 0));
     // the timed sweeps counted iterations and wrote maxima of their own
@@ -2116,7 +2166,7 @@ qesb_status solve_impl(qesb_handle *h, int itermax, float *u, float *v, float *w
   h->last_pre_iterations = 0;
   h->sweeps_timed = false;
   if (itermax > 0) {
-    if (resident) CKS(run_iterations_resident(h, !packed, itermax));
+    if (resident) CKS(run_iterations_resident(h, sch, !packed, itermax));
     else if (split) CKS(run_iterations_sweep(h, kSweepVariants[vi - kSplitVariant], itermax));
     else if (var) CKS(run_iterations_tiled(h, *var, itermax));
     else CKS(run_iterations_full(h, itermax));
@@ -2307,6 +2357,9 @@ qesb_status qesb_create(const qesb_grid *grid, float tol, int device, qesb_handl
     if (cudaMemset(h->d_pc[q], 0, np * sizeof(float)) != cudaSuccess) return fail(qesb_fail(QESB_ERR_CUDA, "cudaMemset failed"));
   if (cudaMemcpy(h->d_dz, h->dz.data(), sizeof(float) * G.Z, cudaMemcpyHostToDevice) != cudaSuccess)
     return fail(qesb_fail(QESB_ERR_CUDA, "cudaMemcpy dz failed"));
+  // room for the resident solve of this grid, so that no solve allocates; without it the solves take the sweeps
+  if (res_plan_of(h, G, res_ctas(device)).nty > 0)
+    res_reserve(h, {res_size(G)}, res_schedule(h->rlist.plans, {res_size(G)}, res_ctas(device)));
   (void)nc;
   (void)nf;
 #undef TRY
@@ -2843,8 +2896,12 @@ qesb_status qesb_solve_batch(qesb_handle *const *hs, int n, int itermax, float *
   // domains solved by the resident kernel, and by the list sweeps
   std::vector<qesb_handle *> res;
   std::vector<int> res_of, str_of;  // batch indices
-  const ResChoice choice = batch_choice(h0, hs, n, itermax);
-  const std::vector<char> &is_res = choice.is_res;
+  ResChoice choice = batch_choice(h0, hs, n, itermax);
+  std::vector<char> &is_res = choice.is_res;
+  std::vector<ResSize> sizes;
+  for (int i = 0; i < n; ++i)
+    if (is_res[i]) sizes.push_back(res_size(hs[i]->G));
+  if (!sizes.empty() && !res_reserve(h0, sizes, choice.sched)) is_res.assign(n, 0);
   for (int i = 0; i < n; ++i) {
     if (is_res[i]) {
       res.push_back(hs[i]);

@@ -274,3 +274,51 @@ def test_a_wait_limit_bounds_an_exchange_and_not_the_solve():
     assert all(x["iterations"] == n and x["ms_sor"] > 30.0 for x in st)
     w = ws[2]
     np.testing.assert_array_equal(lam, O.sor(w.domain, w, O.divergence(w.domain, w), -1.0, n)[0])
+
+
+def test_the_first_solve_of_a_handle_allocates_nothing():
+    import torch
+
+    w = _city(130, 131, 33)
+    d = w.domain
+    out = [torch.zeros(d.numFaceCentered(), device="cuda") for _ in range(3)]
+    for _ in range(2):  # the first handle's solve loads the kernels
+        with qesb.Solver_B200(d, 1e-9) as s:
+            s.set_inputs(w)
+            torch.cuda.synchronize()
+            free = torch.cuda.mem_get_info()[0]
+            s.solve_device(5, *[t.data_ptr() for t in out])
+            torch.cuda.synchronize()
+            used = free - torch.cuda.mem_get_info()[0]
+    assert used == 0
+
+
+def test_full_coefficients_without_room_for_their_split_copies():
+    """79 MB of copies that only the resident solve needs, on a GPU with 32 MB
+    free: the inputs are taken and solved without it."""
+    import torch
+
+    w0 = _city(200, 180, 60)
+    w = _cut(_city(200, 180, 60))
+    d = w.domain
+    out = [torch.zeros(d.numFaceCentered(), device="cuda") for _ in range(3)]
+    L = O.sor(d, w, O.divergence(d, w), 1e-9, 5)[0]
+    with qesb.Solver_B200(d, 1e-9) as s:
+        s.set_option("variant", 0)
+        s.set_inputs(w)
+        s.solve_device(5, *[t.data_ptr() for t in out])  # loads the kernels
+    with qesb.Solver_B200(d, 1e-9) as s:
+        s.set_inputs(w0)  # allocates the handle's own copy of the inputs
+        torch.cuda.empty_cache()
+        full = torch.empty(torch.cuda.mem_get_info()[0] - (32 << 20), dtype=torch.uint8, device="cuda")
+        for _ in range(2):
+            s.resetLambda()
+            s.set_inputs(w)
+            st = s.solve_device(5, *[t.data_ptr() for t in out])
+            assert (st["iterations"], st["path"]) == (5, 0)
+            np.testing.assert_array_equal(s.lambda_, L)
+            for t, a in zip(out, O.correct(d, w, L)):
+                np.testing.assert_array_equal(t.cpu().numpy(), a)
+            del full
+            torch.cuda.empty_cache()
+            full = None
