@@ -1816,15 +1816,24 @@ qesb_status run_iterations_sweep(qesb_handle *h, const SweepVariant &sv, int ite
 // ---------------------------------------------------------------------------
 __global__ void k_res_stamp(ResCtl *ctl) { ctl->t0 = global_ns(); }
 
-// lambda and R of the padded layout into the split layout, one pass.
+// lambda and R of the padded layout into the split layout, one pass. With the
+// window rule, wacc receives the first window's drift of the boundary cells,
+// which the resident kernel leaves out: none, or NaN where one is not finite,
+// and on the full-coefficient path (mirror) the ground plane's rim, which the
+// first iteration's mirror moves to plane 1's values.
 __global__ void k_res_to_split(DevGrid G, SplitGeom S, const float *__restrict__ lam, const float *__restrict__ R,
-                               float *__restrict__ lam_s, float *__restrict__ R_s)
+                               float *__restrict__ lam_s, float *__restrict__ R_s, double *wacc, bool mirror)
 {
   const int j = blockIdx.y, k = blockIdx.z;
   for (int i = threadIdx.x + blockIdx.x * blockDim.x; i < G.X; i += gridDim.x * blockDim.x) {
     const long d = ((i + j + k) & 1) * S.CS + S.row(j, k, G.Y) + (i >> 1), p = G.pad(i, j, k);
-    lam_s[d] = lam[p];
+    const float v = lam[p];
+    lam_s[d] = v;
     R_s[d] = R[p];
+    if (wacc && (i == 0 || i == G.X - 1 || j == 0 || j == G.Y - 1 || k == G.Z - 1)) {
+      const double m = fabs((double)(mirror && k == 0 ? lam[G.pad(i, j, 1)] : v) - (double)v);
+      if (m != 0.0) atomic_max_nonneg(wacc, m);
+    }
   }
 }
 
@@ -2042,8 +2051,8 @@ qesb_status res_enqueue(qesb_handle *lead, const std::vector<qesb_handle *> &hs,
     }
   CKS(wb.flush());
   for (qesb_handle *h : hs)
-    k_res_to_split<<<row_grid(h->G, h->G.Y, h->G.Z, h->G.X), 256, 0, s>>>(h->G, h->S, h->d_lam, h->d_R, h->d_lam_s,
-                                                                         h->d_R_s);
+    k_res_to_split<<<row_grid(h->G, h->G.Y, h->G.Z, h->G.X), 256, 0, s>>>(
+        h->G, h->S, h->d_lam, h->d_R, h->d_lam_s, h->d_R_s, h->win_k > 0 ? &h->d_rsync->wacc[0] : nullptr, full);
   CKS(copy_words(L.blk, L.stage_dev, o_dom + sizeof(ResDomain) * (size_t)n, s));
   k_res_stamp<<<1, 1, 0, s>>>(reinterpret_cast<ResCtl *>(L.blk));
   CK(cudaEventRecord(lead->evs[0], s));

@@ -322,3 +322,42 @@ def test_full_coefficients_without_room_for_their_split_copies():
             del full
             torch.cuda.empty_cache()
             full = None
+
+
+@pytest.mark.parametrize("variant", [-1, 18])
+def test_first_window_counts_the_ground_planes_rim(variant):
+    """Full coefficients, a start whose ground plane is not plane 1's mirror on
+    the rim alone: the mirror of the first iteration moves those cells by more
+    than the window's tolerance, which all others meet at once."""
+    w = _city(47, 41, 20)
+    d = w.domain
+    R = O.divergence(d, w)
+    lam0 = O.sor(d, w, R, 1e-9, 60)[0].reshape(21, 41, 47).copy()
+    lam0[0, 0, 7] += np.float32(5.0)
+    lam0[0, 9, 46] -= np.float32(4.0)
+    with qesb.Solver_B200(d, 1e-9) as s:
+        s.set_option("path", 0)
+        s.set_option("variant", variant)
+        s.set_window_rule(4, 3.0)
+        s.lambda_ = lam0.ravel()
+        st = s.solve(w, 200)
+        L, it, stop, drift = O.sor_window(d, w, R, 1e-9, 200, 4, 3.0, lam=lam0.ravel())
+        assert (st["iterations"], st["converged"], st["window_drift"]) == (it, stop, drift) and it == 8
+        np.testing.assert_array_equal(s.lambda_, L)
+
+
+@pytest.mark.parametrize("path,variant", [(1, -1), (1, 18), (0, -1), (0, 0)])
+def test_window_rule_refuses_a_boundary_that_is_not_a_number(path, variant):
+    """A cell on an edge of the box, which no other cell reads."""
+    w = _city(47, 41, 20)
+    lam0 = np.zeros((21, 41, 47), np.float32)
+    lam0[7, 0, 0] = np.nan
+    with qesb.Solver_B200(w.domain, 1e-9) as s:
+        s.set_option("path", path)
+        s.set_option("variant", variant)
+        s.lambda_ = lam0.ravel()
+        st = s.solve(w, 8)
+        assert st["iterations"] == 8
+        s.set_window_rule(4, 1e-3)
+        with pytest.raises(qesb.QesbError, match="NaN"):
+            s.solve(w, 8)
