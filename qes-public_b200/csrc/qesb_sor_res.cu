@@ -733,7 +733,7 @@ __global__ void __launch_bounds__(kResMaxThreads, 1) k_sor_res(ResArgs a)
         mx.dmax = 0.0;
         for (int c = 0; c < 2; ++c) {
           const unsigned mark = t.epoch + 2 * iters + c;
-          const bool ask = F.tol >= 0.0;
+          const bool ask = !(F.tol < 0.0);  // a tolerance below zero is never met
           if (c == 1 && tid == 0) {
             s_thr[par ^ 1] = 0;
             if (tiles > 1 && ask) {

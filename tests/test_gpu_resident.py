@@ -361,3 +361,13 @@ def test_window_rule_refuses_a_boundary_that_is_not_a_number(path, variant):
         s.set_window_rule(4, 1e-3)
         with pytest.raises(qesb.QesbError, match="NaN"):
             s.solve(w, 8)
+
+
+@pytest.mark.parametrize("variant", [-1, 18])
+def test_a_tolerance_that_is_not_a_number_stops_the_loop(variant):
+    """`max_error > tol` does not hold after the first iteration."""
+    w = _city(47, 41, 20)
+    with qesb.Solver_B200(w.domain, float("nan")) as s:
+        s.set_option("variant", variant)
+        st = s.solve(w, 30)
+        assert (st["iterations"], st["converged"]) == (1, 1)
