@@ -475,7 +475,8 @@ def workspace_read(path: str) -> "WINDSGeneralData":
 
 def autotune_batch(solvers) -> tuple[int, list[float]]:
     """qesb_autotune_batch: times every sweep launch shape on the domain list
-    qesb_solve_batch would run for these solvers (inputs set), keeps the
+    qesb_solve_batch would run for these solvers (inputs set; without those it
+    solves with lambda resident, unless that is all), keeps the
     fastest as solvers[0]'s "batch_variant" option, and returns it with each
     shape's microseconds per iteration over the list (0 for the fused tile
     shapes, which batches do not use)."""
