@@ -661,7 +661,7 @@ __global__ void __launch_bounds__(kResMaxThreads, 1) k_sor_res(ResArgs a)
         if (!res_wait(&sy->bar, s_target, limit, a.ctl)) s_bad = 1;
       }
     };
-    if (D.alias) {
+    if (FULL && D.alias) {
       // every CTA has read its part of the start: the CTA clears its slots of what lies there (lambda, or an earlier
       // solve's words, which carry the same marks), before any neighbour asks for them
       if (tid == 0) meet();
@@ -806,12 +806,11 @@ __global__ void __launch_bounds__(kResMaxThreads, 1) k_sor_res(ResArgs a)
             atomicMax(reinterpret_cast<unsigned long long *>(&s_win), (unsigned long long)__double_as_longlong(dm));
           __syncthreads();
           if (tid == 0) {
-            const int slot = windows % 3, next = (windows + 1) % 3;
-            if (s_win != 0.0) atomic_max_nonneg(&sy->wacc[slot], s_win);
-            // the next window's slot: its last readers arrived at the barrier before, its next writers leave this one
-            if (rank == 0) *reinterpret_cast<volatile double *>(&sy->wacc[next]) = 0.0;
+            if (s_win != 0.0) atomic_max_nonneg(&sy->wacc[windows & 3], s_win);
             meet();
-            s_win = *reinterpret_cast<volatile double *>(&sy->wacc[slot]);
+            s_win = *reinterpret_cast<volatile double *>(&sy->wacc[windows & 3]);
+            // the slot after the next: its last readers arrived at this barrier, its next writers leave the next one
+            if (rank == 0) *reinterpret_cast<volatile double *>(&sy->wacc[(windows & 3) ^ 2]) = 0.0;
           }
           __syncthreads();
           if (s_bad) return;

@@ -27,7 +27,7 @@ struct alignas(128) ResSync {
   unsigned long long pad_[14];
   unsigned cert;           // number of the last iteration proven not to stop
   unsigned beat;           // the first CTA's iteration number, for CTAs of the group that wait for the next domain
-  double wacc[3];          // window rule: max|lambda - snapshot|, windows in turn (the first starts from the boundary's)
+  double wacc[4];          // window rule: max|lambda - snapshot|, windows in turn (the first starts from the boundary's)
 };
 
 struct ResDomain {
