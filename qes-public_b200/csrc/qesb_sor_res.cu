@@ -31,12 +31,17 @@
 // row code has no divergent branch: those cost more than its sums.
 //
 // Measured (B200, us an iteration of one domain, against the fastest streaming
-// shape): 40 x 40 x 20 5.7 (8.6), 100 x 100 x 50 7.6 (12.7), 200 x 180 x 60 10.0
-// (18.6), 256 x 256 x 64 14.2 (21.0). A half-sweep of the last takes about 7 us:
-// 3 for the rows (issue and shared-memory latency; their FP32 operations alone
-// would take 0.9), 0.5 for the wall cells, the rest for the faces: 47 KB in and
-// out of L2 per CTA and the wait for the slowest neighbour. Small domains are all
-// latency: two exchanges of about 1.2 us each.
+// shape): 40 x 40 x 20 5.6 (8.6), 100 x 100 x 50 7.2 (12.7), 200 x 180 x 60 10.2
+// (18.6), 256 x 256 x 64 13.7 (21.0). A half-sweep of the last takes about 7 us;
+// the FP32 operations of its rows alone would take 0.9. 16 warps an SM issue in 47 %
+// of the cycles (rows: fixed and shared-memory latency); a third of their time is
+// the CTA barriers and the loads of faces and of streamed R: 47 KB in and out of L2
+// per CTA and the wait for the slowest neighbour. Small domains are all latency:
+// two exchanges of about 1.2 us each.
+//
+// The kernel sits at the limit of 128 registers a thread: code added beside the
+// rows (two more slots of the window rule by remainder, the alias path in the
+// wall-mask kernel) has cost 4 % at 100 x 100 x 50.
 //
 // FULL: every cell has its own six coefficients (no wall mask): they stream from
 // L2, 28 B a cell with omega / (their sum), while lambda still stays here. An
